@@ -60,7 +60,7 @@ __device__ __forceinline__ bool solve_control(EcgStepStats* __restrict__ st, con
 }
 
 template <int RK, int LIM, int H, int WPB>
-__global__ void __launch_bounds__(WPB * 32, 12 / WPB)
+__global__ void __launch_bounds__(WPB * 32, march::kStagedWarps<RK> / WPB)
 fv_batch_kernel(const EcgBatchSolve* __restrict__ solves, EcgStepStats* __restrict__ stats,
                 unsigned long long* __restrict__ degenerate_total, const int* __restrict__ max_step,
                 const EcgBatchCtl ctl)
@@ -95,7 +95,7 @@ fv_batch_kernel(const EcgBatchSolve* __restrict__ solves, EcgStepStats* __restri
     march::MarchAcc acc;
     acc.init();
     if (c0 < S.p.g.nx)
-      march::march_strip_staged<RK, LIM, true>(S.p, S.u[par], S.u[par ^ 1], c0, j0, H, s_dt,
+      march::march_strip_staged<RK, LIM>(S.p, S.u[par], S.u[par ^ 1], c0, j0, H, s_dt,
                                                ctl.count_degenerate != 0, acc, ring[warp]);
     const int deg = block_commit<WPB * 32>(red, acc.kmax, acc.krho, acc.kp, acc.nonfinite, acc.degenerate,
                                            &stats[3 * s + ctl.acc_slot]);

@@ -53,6 +53,26 @@ __device__ __forceinline__ double fsound(double rho, double p, double g)
   return t * frsqrt(q);
 }
 
+// limited_slope (state_primitives.hpp:57-91) with one sign test: for
+// one-sided differences of one sign the nested minmods pick by magnitude
+// alone, and the van Leer quotient takes the refined reciprocal.
+__device__ __forceinline__ double slope_f(double bk, double fw, int lim)
+{
+  const double prod = bk * fw;
+  double s;
+  if (lim == 1) {
+    const double c = 0.5 * (bk + fw);
+    const double t = fabs(2.0 * bk) < fabs(c) ? 2.0 * bk : c;
+    s = fabs(t) < fabs(2.0 * fw) ? t : 2.0 * fw;
+  } else if (lim == 2) {
+    const double d = bk + fw;
+    s = fabs(d) <= 1.0e-14 ? 0.0 : 2.0 * prod * frcp(d);
+  } else {
+    s = fabs(bk) < fabs(fw) ? bk : fw;
+  }
+  return prod <= 0.0 ? 0.0 : s;
+}
+
 __device__ __forceinline__ Prim to_prim_f(const Cons& c, double g)
 {
   const double inv_rho = frcp(c.rho);
@@ -128,12 +148,12 @@ __device__ __forceinline__ Cons hllc_f(const Prim& l, const Prim& r, int axis, d
   return rusanov_i(l, r, axis, g, inv_gm1);
 }
 
-// 0 < x < 1e300 by one unsigned integer compare of the bit pattern (positive
-// doubles order like their bits; zero, negatives, NaN and huge values fail).
+// Normal and below about 1e300, by one unsigned compare of the high word
+// (positive doubles order like their bits; zero, denormals, negatives, NaN
+// and huge values fail).
 __device__ __forceinline__ bool pos_normal_range(double x)
 {
-  constexpr unsigned long long kHi = 0x7E37E43C8800759CULL;  // bits of 1.0e300
-  return static_cast<unsigned long long>(__double_as_longlong(x)) - 1ULL < kHi - 1ULL;
+  return static_cast<unsigned>(__double2hiint(x)) - 0x00100000u < 0x7E37E43Cu - 0x00100000u;
 }
 
 // fsound for whole warps: the rsqrt path, and the IEEE formula only when some
@@ -150,97 +170,89 @@ __device__ __forceinline__ double fsound_w(double rho, double p, double g)
   return c;
 }
 
-// hllc_flux of hllc_f without divergent branches: every lane evaluates the
-// star-state flux of its upwind side, supersonic faces select the plain
-// physical flux, and the Rusanov fallback (the three degenerate cases of
-// reconstruction_fluxes.hpp:151-210) runs only when some lane of the warp
-// needs it.  deg: that fallback was taken.
-__device__ __forceinline__ Cons hllc_w(const Prim& l, const Prim& r, int axis, double g, double inv_gm1, bool& deg)
-{
-  const double unl = normal_vel(l, axis), unr = normal_vel(r, axis);
-  const double cl = fsound_w(l.rho, l.p, g), cr = fsound_w(r.rho, r.p, g);
-  const double sl = smin(unl - cl, unr - cr), sr = smax(unl + cl, unr + cr);
-  const bool ordered = sl < sr;
-  const bool sup_l = sl >= 0.0, sup_r = sr <= 0.0;
-  const bool supersonic = ordered && (sup_l || sup_r);
-  const double al = l.rho * (sl - unl), ar = r.rho * (sr - unr);
-  const double den = al - ar;
-  const double sm = fdiv(r.p - l.p + al * unl - ar * unr, den);
-  const double lsd = sl - sm, rsd = sr - sm;
-  deg = !ordered || (!supersonic && (fabs(den) <= 1.0e-12 || fabs(lsd) <= 1.0e-12 || fabs(rsd) <= 1.0e-12));
-  const bool left = supersonic ? sup_l : sm >= 0.0;
-  const Prim q = left ? l : r;
-  const double s = left ? sl : sr, un = left ? unl : unr, a = left ? al : ar;
-  const Cons u = to_cons_f(q, inv_gm1);
-  const Cons f = pflux(q, u, axis);
-  const double ps = 0.5 * (l.p + al * (sm - unl) + r.p + ar * (sm - unr));
-  const double inv_sd = frcp(left ? lsd : rsd);
-  const double rs = a * inv_sd;
-  const double es = ((s - un) * u.E - q.p * un + ps * sm) * inv_sd;
-  const double tang = axis == 0 ? q.v : q.u;
-  const double smx = axis == 0 ? rs * sm : rs * tang;
-  const double smy = axis == 0 ? rs * tang : rs * sm;
-  Cons out;
-  out.rho = supersonic ? f.rho : fma(s, rs - u.rho, f.rho);
-  out.mx = supersonic ? f.mx : fma(s, smx - u.mx, f.mx);
-  out.my = supersonic ? f.my : fma(s, smy - u.my, f.my);
-  out.E = supersonic ? f.E : fma(s, es - u.E, f.E);
-  if (__any_sync(0xffffffffu, deg)) {
-    const Cons rf = rusanov_i(l, r, axis, g, inv_gm1);
-    if (deg) out = rf;
-  }
-  return out;
-}
-
-// Sound speed on the rsqrt path only; `bad` marks states outside (0, 1e300)
-// whose speed must come from the IEEE formula instead.
-__device__ __forceinline__ double fsound_core(double rho, double p, double g, bool& bad)
+// Sound speed on the rsqrt path only, and its inverse sqrt(rho / (g p)) from
+// the same square root; `bad` marks states outside (0, 1e300) whose speed must
+// come from the IEEE formula instead.
+struct Sound {
+  double c, inv;
+};
+__device__ __forceinline__ Sound sound_core(double rho, double p, double g, bool& bad)
 {
   const double t = g * p;
   const double q = t * rho;
   bad = !pos_normal_range(q);
-  return t * frsqrt(q);
+  const double y = frsqrt(q);
+  return Sound{t * y, rho * y};
 }
 
-// hllc_w without any warp vote: the branch-free HLLC flux of states whose
-// sound speeds are on the rsqrt path and whose star state is not degenerate.
-// `fallback` marks the faces that must be recomputed by hllc_f instead
-// (degenerate star state or a sound speed off the rsqrt path), so two faces
-// can be evaluated back to back and repaired by one vote.
-__device__ __forceinline__ Cons hllc_core(const Prim& l, const Prim& r, int axis, double g, double inv_gm1,
+// min(max(|u_l|/c_l, |u_r|/c_r), 1) from the squared speeds and the inverse
+// sound speeds: one square root for both sides, none for a state at rest.
+__device__ __forceinline__ double mach_limit(double sp2l, double icl, double sp2r, double icr)
+{
+  const double m2 = smax(sp2l * (icl * icl), sp2r * (icr * icr));
+  return m2 < 1.0 ? (m2 > 1.0e-300 ? m2 * frsqrt(m2) : 0.0) : 1.0;
+}
+
+// hllc_flux of hllc_f (LM: after lowmach_f's correction of the two states,
+// whose sound speeds the flux shares) without branches or votes: the flux of
+// faces whose sound speeds are on the rsqrt path and whose star state is not
+// degenerate.  `fallback` marks the faces that hllc_f must recompute
+// (degenerate star state, a sound speed off the rsqrt path or, for LM, below
+// the floor of the Mach numbers), so that a warp evaluates two faces back to
+// back and repairs them after one vote.
+//
+// The star flux F_K + s_K (U*_K - U_K) is evaluated in its collapsed form: by
+// the jump conditions across s_K it equals
+//   m = rho*_K s_M,  (m, m s_M + p*, m u_t, s_M (E*_K + p*)),
+// which needs neither the side's conserved momenta and physical flux nor the
+// four differences, and has no cancellation between the two at low Mach.  A
+// supersonic face is the same expression with s_M = u_n and p* = p.
+// The step is bound by FP64 issue and latency, so operations are time: 2560x640
+// HLLC 69.9 -> 67.1 us, 1021x509 low-Mach HLLC with van Leer slopes (whose
+// quotient and Mach numbers took IEEE divisions and branches) 73.4 -> 42.6 us.
+template <bool LM>
+__device__ __forceinline__ Cons hllc_core(const Prim& ql, const Prim& qr, int axis, double g, double inv_gm1,
                                           bool& fallback)
 {
-  const double unl = normal_vel(l, axis), unr = normal_vel(r, axis);
+  double unl = axis == 0 ? ql.u : ql.v, utl = axis == 0 ? ql.v : ql.u;
+  double unr = axis == 0 ? qr.u : qr.v, utr = axis == 0 ? qr.v : qr.u;
   bool bl, br;
-  const double cl = fsound_core(l.rho, l.p, g, bl), cr = fsound_core(r.rho, r.p, g, br);
+  const Sound sndl = sound_core(ql.rho, ql.p, g, bl), sndr = sound_core(qr.rho, qr.p, g, br);
+  const double cl = sndl.c, cr = sndr.c;
+  bool off = bl || br;
+  if (LM) {
+    off = off || !(cl > 1.0e-12) || !(cr > 1.0e-12);
+    const double z = mach_limit(unl * unl + utl * utl, sndl.inv, unr * unr + utr * utr, sndr.inv);
+    const double hz = 0.5 * z;
+    const double an = 0.5 * (unl + unr), at = 0.5 * (utl + utr);
+    const double dn = hz * (unl - unr), dt = hz * (utl - utr);
+    unl = an + dn;
+    unr = an - dn;
+    utl = at + dt;
+    utr = at - dt;
+  }
   const double sl = smin(unl - cl, unr - cr), sr = smax(unl + cl, unr + cr);
   const bool ordered = sl < sr;
   const bool sup_l = sl >= 0.0, sup_r = sr <= 0.0;
-  const bool supersonic = ordered && (sup_l || sup_r);
-  const double al = l.rho * (sl - unl), ar = r.rho * (sr - unr);
+  const bool supersonic = sup_l || sup_r;
+  const double al = ql.rho * (sl - unl), ar = qr.rho * (sr - unr);
   const double den = al - ar;
-  const double sm = fdiv(r.p - l.p + al * unl - ar * unr, den);
-  const double lsd = sl - sm, rsd = sr - sm;
-  const bool deg = !ordered || (!supersonic && (fabs(den) <= 1.0e-12 || fabs(lsd) <= 1.0e-12 || fabs(rsd) <= 1.0e-12));
-  fallback = deg || bl || br;
-  const bool left = supersonic ? sup_l : sm >= 0.0;
-  const Prim q = left ? l : r;
-  const double s = left ? sl : sr, un = left ? unl : unr, a = left ? al : ar;
-  const Cons u = to_cons_f(q, inv_gm1);
-  const Cons f = pflux(q, u, axis);
-  const double ps = 0.5 * (l.p + al * (sm - unl) + r.p + ar * (sm - unr));
-  const double inv_sd = frcp(left ? lsd : rsd);
-  const double rs = a * inv_sd;
-  const double es = ((s - un) * u.E - q.p * un + ps * sm) * inv_sd;
-  const double tang = axis == 0 ? q.v : q.u;
-  const double smx = axis == 0 ? rs * sm : rs * tang;
-  const double smy = axis == 0 ? rs * tang : rs * sm;
-  Cons out;
-  out.rho = supersonic ? f.rho : fma(s, rs - u.rho, f.rho);
-  out.mx = supersonic ? f.mx : fma(s, smx - u.mx, f.mx);
-  out.my = supersonic ? f.my : fma(s, smy - u.my, f.my);
-  out.E = supersonic ? f.E : fma(s, es - u.E, f.E);
-  return out;
+  const double sm0 = fdiv(qr.p - ql.p + al * unl - ar * unr, den);
+  const bool deg =
+      !ordered || (!supersonic && (fabs(den) <= 1.0e-12 || fabs(sl - sm0) <= 1.0e-12 || fabs(sr - sm0) <= 1.0e-12));
+  fallback = deg || off;
+  const bool left = supersonic ? sup_l : sm0 >= 0.0;
+  const double rho = left ? ql.rho : qr.rho, un = left ? unl : unr, ut = left ? utl : utr, p = left ? ql.p : qr.p;
+  const double s = left ? sl : sr;
+  const double sm = supersonic ? un : sm0;
+  const double ps = supersonic ? p : 0.5 * (fma(al, sm0 - unl, ql.p) + fma(ar, sm0 - unr, qr.p));
+  const double inv_sd = frcp(s - sm);
+  const double d = s - un;
+  const double m = rho * d * inv_sd * sm;
+  const double E = fma(p, inv_gm1, 0.5 * rho * fma(un, un, ut * ut));
+  const double es = (d * E - p * un + ps * sm) * inv_sd;
+  const double mn = fma(m, sm, ps), mt = m * ut;
+  return Cons{m, axis == 0 ? mn : mt, axis == 0 ? mt : mn, sm * (es + ps)};
 }
 
 // rusanov_i on the rsqrt path; `fallback` as for hllc_core.
@@ -250,7 +262,7 @@ __device__ __forceinline__ Cons rusanov_core(const Prim& l, const Prim& r, int a
   const Cons ul = to_cons_f(l, inv_gm1), ur = to_cons_f(r, inv_gm1);
   const Cons fl = pflux(l, ul, axis), fr = pflux(r, ur, axis);
   bool bl, br;
-  const double cl = fsound_core(l.rho, l.p, g, bl), cr = fsound_core(r.rho, r.p, g, br);
+  const double cl = sound_core(l.rho, l.p, g, bl).c, cr = sound_core(r.rho, r.p, g, br).c;
   fallback = bl || br;
   const double sm = smax(fabs(normal_vel(l, axis)) + cl, fabs(normal_vel(r, axis)) + cr);
   const double hs = 0.5 * sm;
@@ -344,74 +356,70 @@ static __device__ __noinline__ Cons xie_f(const Prim l, const Prim r, int axis, 
 
 // xie_f without branches: the flux of a face whose states take none of
 // xie_f's exits (sound speeds on the rsqrt path, ordered wave speeds, and for
-// a subsonic face no degenerate denominator, square roots on their fast path
-// and a finite result), evaluated with xie_f's arithmetic in xie_f's order;
-// a supersonic face selects the upwind physical flux as xie_f returns it.
-// `fallback` marks the faces xie_f must evaluate instead (the caller does so
-// after one warp vote); deg: the HLLC degeneracy test, valid without fallback.
+// a subsonic face no degenerate denominator, densities and Roe sound speed on
+// the fast path and a finite result).  `fallback` marks the faces xie_f must
+// evaluate instead (the caller does so after one warp vote; the thresholds
+// here are a shade wider than xie_f's, which decides).  No face that stays is
+// degenerate for the HLLC test: its middle speed is this one.
+//
+// The algebra of xie_f with its divisions folded: enthalpies and specific
+// energies from the squared sound speeds (c^2 = g p / rho), the density
+// weights sqrt(rho_K) / (sqrt(rho_l) + sqrt(rho_r)) from one square root of
+// the product, the Mach blend from the inverse speeds, rs (p / a) = p / s_d,
+// and a supersonic face as the same expression with ss = q_n, p*** = p* = p
+// and no pressure diffusion: 6 square roots and 5 reciprocals in place of 7
+// and 11.  2560x640 on strips 138 -> 120 us, 256x256 on tiles 12.7 -> 11.3 us.
 __device__ __forceinline__ Cons xie_core(const Prim& l, const Prim& r, int axis, double g, double inv_gm1,
-                                         double sensor, bool& fallback, bool& deg)
+                                         double f, bool& fallback)
 {
-  const double ql = normal_vel(l, axis), qr = normal_vel(r, axis);
+  constexpr double kTiny = 1.001e-12;
+  const double unl = axis == 0 ? l.u : l.v, utl = axis == 0 ? l.v : l.u;
+  const double unr = axis == 0 ? r.u : r.v, utr = axis == 0 ? r.v : r.u;
   const double pl = l.p, pr = r.p;
   bool bl, br;
-  const double cl = fsound_core(l.rho, pl, g, bl), cr = fsound_core(r.rho, pr, g, br);
-  const double sl = smin(ql - cl, qr - cr), sr = smax(ql + cl, qr + cr);
+  const Sound sndl = sound_core(l.rho, pl, g, bl), sndr = sound_core(r.rho, pr, g, br);
+  const double cl = sndl.c, cr = sndr.c;
+  const double sl = smin(unl - cl, unr - cr), sr = smax(unl + cl, unr + cr);
   const bool ordered = sl < sr;
   const bool sup_l = sl >= 0.0, sup_r = sr <= 0.0;
   const bool supersonic = sup_l || sup_r;
-  const double al = l.rho * (sl - ql), ar = r.rho * (sr - qr);
+  const double al = l.rho * (sl - unl), ar = r.rho * (sr - unr);
   const double ad = ar - al;
   const double inv_ad = frcp(ad);
-  const double sm = (r.p - l.p + al * ql - ar * qr) * -inv_ad;
-  deg = !supersonic && (fabs(sl - sm) <= 1.0e-12 || fabs(sr - sm) <= 1.0e-12);
-  const double ss = (ar * qr - al * ql + pl - pr) * inv_ad;
-  const double dl = sl - ss, dr = sr - ss;
-  const Cons ul = to_cons_f(l, inv_gm1), ur = to_cons_f(r, inv_gm1);
-  const double ps = (ar * pl - al * pr - al * ar * (ql - qr)) * inv_ad;
-  const double srl = l.rho * frsqrt(l.rho), srr = r.rho * frsqrt(r.rho);
-  const double rd = srl + srr;
-  const double ird = frcp(rd);
-  const double uh = (srl * l.u + srr * r.u) * ird;
-  const double vh = (srl * l.v + srr * r.v) * ird;
-  const double qh = axis == 0 ? uh : vh;
-  const double hl = fdiv(ul.E + pl, l.rho), hr = fdiv(ur.E + pr, r.rho);
-  const double hh = (srl * hl + srr * hr) * ird;
-  const double c2 = (g - 1.0) * (hh - 0.5 * (uh * uh + vh * vh));
-  const double ch = c2 * frsqrt(c2);
-  const double mh = fdiv(qh, smax(ch, 1.0e-12));
-  // |u| of a state at rest is fsqrt's sqrt(0) = 0: kept on the fast path
-  const double sp2l = l.u * l.u + l.v * l.v, sp2r = r.u * r.u + r.v * r.v;
-  const bool okl = pos_normal_range(sp2l), okr = pos_normal_range(sp2r);
-  const double spl = okl ? sp2l * frsqrt(sp2l) : sp2l, spr = okr ? sp2r * frsqrt(sp2r) : sp2r;
-  const double th = clamp01(smax(fdiv(spl, smax(cl, 1.0e-12)), fdiv(spr, smax(cr, 1.0e-12))));
-  const double f = clamp01(sensor);
-  const double pss = th * ps + (1.0 - th) * 0.5 * (pl + pr);
-  const double psss = f * pss + (1.0 - f) * ps;
-  const double bp = fdiv((f - 1.0) * sl * sr * (pr - pl), (sr - sl) * (c2 * (1.0 + fabs(mh))));
-  const double nxv = axis == 0 ? 1.0 : 0.0, nyv = axis == 1 ? 1.0 : 0.0;
-  const bool left = ss >= 0.0;
-  const Prim q = left ? l : r;
-  const double qn = left ? ql : qr;
-  const double a = left ? al : ar;
-  const double rs = fdiv(a, left ? dl : dr);
-  const double e = left ? fdiv(ul.E, l.rho) : fdiv(ur.E, r.rho);
-  const double es = e + (ss - qn) * (ss + fdiv(left ? pl : pr, a));
+  const double ss0 = (ar * unr - al * unl + pl - pr) * inv_ad;
+  const double ps0 = (ar * pl - al * pr - al * ar * (unl - unr)) * inv_ad;
+  // Roe averages
+  const double rr = l.rho * r.rho;
+  const double root = r.rho * frsqrt(rr);  // sqrt(rho_r / rho_l)
+  const double wl = frcp(1.0 + root), wr = root * wl;
+  const double nh = wl * unl + wr * unr, th = wl * utl + wr * utr;
+  const double sp2l = unl * unl + utl * utl, sp2r = unr * unr + utr * utr;
+  const double c2l = cl * cl, c2r = cr * cr;
+  const double hh = wl * fma(c2l, inv_gm1, 0.5 * sp2l) + wr * fma(c2r, inv_gm1, 0.5 * sp2r);
+  const double v2h = nh * nh + th * th;
+  const double c2 = (g - 1.0) * (hh - 0.5 * v2h);
+  const double mh = fabs(nh) * frsqrt(c2);
+  const double blend = mach_limit(sp2l, sndl.inv, sp2r, sndr.inv);
+  const double pss = blend * ps0 + (1.0 - blend) * 0.5 * (pl + pr);
+  const double psss0 = f * pss + (1.0 - f) * ps0;
+  const double bp0 = fdiv((f - 1.0) * sl * sr * (pr - pl), (sr - sl) * (c2 * (1.0 + mh)));
+  const bool left = supersonic ? sup_l : ss0 >= 0.0;
+  const double rho = left ? l.rho : r.rho, un = left ? unl : unr, ut = left ? utl : utr, p = left ? pl : pr;
+  const double s = left ? sl : sr, c2k = left ? c2l : c2r, sp2 = left ? sp2l : sp2r;
+  const double ss = supersonic ? un : ss0, ps = supersonic ? p : ps0, psss = supersonic ? p : psss0;
+  const double bp = supersonic ? 0.0 : bp0;
+  const double inv_sd = frcp(s - ss);
+  const double rs = rho * (s - un) * inv_sd;
+  const double e = fma(c2k, inv_gm1 / g, 0.5 * sp2);
   const double rss = rs * ss;
-  const Cons sub{rss + bp, rss * (q.u + nxv * (ss - qn)) + nxv * psss + bp * uh,
-                 rss * (q.v + nyv * (ss - qn)) + nyv * psss + bp * vh,
-                 ss * (rs * es + ps) + 0.5 * bp * (uh * uh + vh * vh)};
-  // xie_f's exits of a subsonic face, and the square roots fsqrt would take
-  // off its rsqrt path (l.rho, r.rho, c2, the speeds; 0 < x < 1e300 there)
-  const bool sub_exit = fabs(ad) <= 1.0e-12 || fabs(dl) <= 1.0e-12 || fabs(dr) <= 1.0e-12 ||
-                        fabs(al) <= 1.0e-12 || fabs(ar) <= 1.0e-12 || !pos_normal_range(l.rho) ||
-                        !pos_normal_range(r.rho) || !(rd > 0.0) || !(c2 > 0.0) || !isfinite(c2) ||
-                        !pos_normal_range(c2) || !(okl || sp2l == 0.0) || !(okr || sp2r == 0.0) ||
-                        !isfinite(sub.rho) || !isfinite(sub.mx) || !isfinite(sub.my) || !isfinite(sub.E);
+  const double mn = fma(rss, ss, psss) + bp * nh, mt = rss * ut + bp * th;
+  const double FE = ss * (rs * e + (ss - un) * fma(p, inv_sd, rss) + ps) + 0.5 * bp * v2h;
+  const bool sub_exit = fabs(ad) <= kTiny || fabs(sl - ss0) <= kTiny || fabs(sr - ss0) <= kTiny ||
+                        fabs(al) <= kTiny || fabs(ar) <= kTiny || !pos_normal_range(rr) || !(l.rho > 0.0) ||
+                        !(cl > kTiny) || !(cr > kTiny) || !(c2 > 1.01e-24) || !(c2 < 1.0e300) ||
+                        !isfinite(FE + mn + mt);
   fallback = bl || br || !ordered || (!supersonic && sub_exit);
-  if (!supersonic) return sub;
-  const Prim& w = sup_l ? l : r;
-  return pflux(w, sup_l ? ul : ur, axis);
+  return Cons{rss + bp, axis == 0 ? mn : mt, axis == 0 ? mt : mn, FE};
 }
 
 // Face pressure ratio of the multiface sensor (reconstruction_fluxes.hpp:390-397):
@@ -486,8 +494,8 @@ fv_fast_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
     for (int k = 0; k < 4; ++k) {
       const double* q = pl[k];
       const double qc = q[c];
-      sl[k * S::SN + e] = second ? limited_slope(qc - q[c - 1], q[c + 1] - qc, lim) : 0.0;
-      sl[(4 + k) * S::SN + e] = second ? limited_slope(qc - q[c - RW], q[c + RW] - qc, lim) : 0.0;
+      sl[k * S::SN + e] = second ? slope_f(qc - q[c - 1], q[c + 1] - qc, lim) : 0.0;
+      sl[(4 + k) * S::SN + e] = second ? slope_f(qc - q[c - RW], q[c + RW] - qc, lim) : 0.0;
     }
   }
   __syncthreads();
@@ -535,8 +543,8 @@ fv_fast_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
       m = smin(m, yr[y * (T + 2) + fx + 1]);
       m = smin(m, yr[(y + 1) * (T + 2) + fx + 1]);
       const double h = clamp01(m);
-      bool fb, deg;
-      Cons f = xie_core(L, Rr, 0, g, inv_gm1, h * h * h, fb, deg);
+      bool fb, deg = false;
+      Cons f = xie_core(L, Rr, 0, g, inv_gm1, h * h * h, fb);
       fb = fb && valid;
       if (__any_sync(0xffffffffu, fb)) {
         if (fb) f = xie_f(L, Rr, 0, g, inv_gm1, h * h * h, deg);
@@ -563,8 +571,8 @@ fv_fast_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
       m = smin(m, xr[(fy + 1) * (T + 1) + x]);
       m = smin(m, xr[(fy + 1) * (T + 1) + x + 1]);
       const double h = clamp01(m);
-      bool fb, deg;
-      Cons f = xie_core(L, Rr, 1, g, inv_gm1, h * h * h, fb, deg);
+      bool fb, deg = false;
+      Cons f = xie_core(L, Rr, 1, g, inv_gm1, h * h * h, fb);
       fb = fb && valid;
       if (__any_sync(0xffffffffu, fb)) {
         if (fb) f = xie_f(L, Rr, 1, g, inv_gm1, h * h * h, deg);

@@ -30,8 +30,8 @@ template <int LIM>
 __device__ __forceinline__ Prim slope3(const Prim& m, const Prim& c, const Prim& p, bool second)
 {
   if (!second) return Prim{0.0, 0.0, 0.0, 0.0};
-  return Prim{limited_slope(c.rho - m.rho, p.rho - c.rho, LIM), limited_slope(c.u - m.u, p.u - c.u, LIM),
-              limited_slope(c.v - m.v, p.v - c.v, LIM), limited_slope(c.p - m.p, p.p - c.p, LIM)};
+  return Prim{fast::slope_f(c.rho - m.rho, p.rho - c.rho, LIM), fast::slope_f(c.u - m.u, p.u - c.u, LIM),
+              fast::slope_f(c.v - m.v, p.v - c.v, LIM), fast::slope_f(c.p - m.p, p.p - c.p, LIM)};
 }
 
 __device__ __forceinline__ Prim plus_half(const Prim& q, const Prim& s)
@@ -41,6 +41,17 @@ __device__ __forceinline__ Prim plus_half(const Prim& q, const Prim& s)
 __device__ __forceinline__ Prim minus_half(const Prim& q, const Prim& s)
 {
   return Prim{fma(-0.5, s.rho, q.rho), fma(-0.5, s.u, q.u), fma(-0.5, s.v, q.v), fma(-0.5, s.p, q.p)};
+}
+
+// One face on its own, every branch taken (the y-face below the first row of a
+// strip, and the faces the branch-free cores send back).
+template <int RK>
+__device__ __forceinline__ Cons face_one(Prim l, Prim r, int axis, double g, double inv_gm1, bool& deg)
+{
+  deg = false;
+  if (RK == ECG_RIEMANN_RUSANOV) return fast::rusanov_f(l, r, axis, g, inv_gm1);
+  if (RK == ECG_RIEMANN_LOWMACH_HLLC) fast::lowmach_f(l, r, g);
+  return fast::hllc_f(l, r, axis, g, inv_gm1, deg);
 }
 
 // The x-face and the y-face of a row, evaluated back to back on the fast
@@ -53,50 +64,37 @@ template <int RK>
 __device__ __forceinline__ bool face_pair(Prim xl, Prim xr, Prim yl, Prim yr, double g, double inv_gm1, Cons& fx,
                                           Cons& fy, bool& deg_x, bool& deg_y)
 {
-  if (RK == ECG_RIEMANN_LOWMACH_HLLC) {
-    fast::lowmach_f(xl, xr, g);
-    fast::lowmach_f(yl, yr, g);
-  }
   bool bx, by;
+  constexpr bool LM = RK == ECG_RIEMANN_LOWMACH_HLLC;
   if (RK == ECG_RIEMANN_RUSANOV) {
     fx = fast::rusanov_core(xl, xr, 0, g, inv_gm1, bx);
     fy = fast::rusanov_core(yl, yr, 1, g, inv_gm1, by);
   } else {
-    fx = fast::hllc_core(xl, xr, 0, g, inv_gm1, bx);
-    fy = fast::hllc_core(yl, yr, 1, g, inv_gm1, by);
+    fx = fast::hllc_core<LM>(xl, xr, 0, g, inv_gm1, bx);
+    fy = fast::hllc_core<LM>(yl, yr, 1, g, inv_gm1, by);
   }
   deg_x = deg_y = false;
   if (__any_sync(0xffffffffu, bx || by)) {
-    if (RK == ECG_RIEMANN_RUSANOV) {
-      if (bx) fx = fast::rusanov_f(xl, xr, 0, g, inv_gm1);
-      if (by) fy = fast::rusanov_f(yl, yr, 1, g, inv_gm1);
-    } else {
-      if (bx) fx = fast::hllc_f(xl, xr, 0, g, inv_gm1, deg_x);
-      if (by) fy = fast::hllc_f(yl, yr, 1, g, inv_gm1, deg_y);
-    }
+    if (bx) fx = face_one<RK>(xl, xr, 0, g, inv_gm1, deg_x);
+    if (by) fy = face_one<RK>(yl, yr, 1, g, inv_gm1, deg_y);
     return true;
   }
   return false;
 }
 
-// One face with the warp-voting flux (faces evaluated one after the other).
+// One face, repaired after a vote of its own (faces evaluated one after the other).
 template <int RK>
 __device__ __forceinline__ Cons face_w(Prim l, Prim r, int axis, double g, double inv_gm1, bool& deg)
 {
+  bool b;
+  constexpr bool LM = RK == ECG_RIEMANN_LOWMACH_HLLC;
+  Cons f = RK == ECG_RIEMANN_RUSANOV ? fast::rusanov_core(l, r, axis, g, inv_gm1, b)
+                                     : fast::hllc_core<LM>(l, r, axis, g, inv_gm1, b);
   deg = false;
-  if (RK == ECG_RIEMANN_RUSANOV) return fast::rusanov_i(l, r, axis, g, inv_gm1);
-  if (RK == ECG_RIEMANN_LOWMACH_HLLC) fast::lowmach_f(l, r, g);
-  return fast::hllc_w(l, r, axis, g, inv_gm1, deg);
-}
-
-// One face on its own (the y-face below the first row of a strip).
-template <int RK>
-__device__ __forceinline__ Cons face_one(Prim l, Prim r, int axis, double g, double inv_gm1, bool& deg)
-{
-  deg = false;
-  if (RK == ECG_RIEMANN_RUSANOV) return fast::rusanov_f(l, r, axis, g, inv_gm1);
-  if (RK == ECG_RIEMANN_LOWMACH_HLLC) fast::lowmach_f(l, r, g);
-  return fast::hllc_f(l, r, axis, g, inv_gm1, deg);
+  if (__any_sync(0xffffffffu, b)) {
+    if (b) f = face_one<RK>(l, r, axis, g, inv_gm1, deg);
+  }
+  return f;
 }
 
 // Reductions of one warp strip over the new state.
@@ -209,7 +207,7 @@ __device__ __forceinline__ void march_strip(const EcgFvParams& P, const double* 
   }
 }
 
-// ---- the staged march: rows reach the warp through shared memory --------
+// ---- the staged march: rows live in shared memory --------------------------
 //
 // Each warp keeps the conserved values of the rows it is about to use in a
 // ring of kRing rows in shared memory (slot = row mod kRing, component planes
@@ -217,16 +215,21 @@ __device__ __forceinline__ void march_strip(const EcgFvParams& P, const double* 
 // the one being converted with cp.async (8 bytes per component, straight
 // from the state, the exact-Dirichlet ring or a slab halo, whichever the
 // ghost policy names); constant ghost states are stored directly.  The load
-// latency of a row is thus hidden behind kAhead rows of flux work without
-// holding registers, and the old state of the updated row is read back from
-// the ring instead of from global memory.  Each lane only reads the slots it
-// wrote itself, so cp.async.wait_group is the only synchronisation.
+// latency of a row is thus hidden behind kAhead rows of flux work, and the
+// old state of the updated row is read back from the ring.
+// A row that has landed is converted once; its velocities and pressure go to a
+// second ring of kPrim rows (the density is the conserved one), from which the
+// lanes read their own column's rows j .. j+2 for the y-slope and their
+// neighbours' row j for the x-slope.  Between rows a lane carries only the
+// y-face below it and the upper face state of its cell.
 constexpr int kRing = 8;
 constexpr int kAhead = 4;
-static_assert(kAhead + 4 <= kRing, "the prologue stages rows j0-2 .. j0+1+kAhead");
+constexpr int kPrim = 4;
+static_assert(kAhead + 4 <= kRing, "rows j-1 .. j+2+kAhead are in the ring");
 
 struct StageRing {
   double v[kRing][4][kLanes];
+  double q[kPrim][3][kLanes];  // u, v, p
 };
 
 __device__ __forceinline__ void cp_async8(unsigned dst, const double* src)
@@ -248,7 +251,7 @@ template <int LIM>
 __device__ __forceinline__ double xface_ratio(double pc, bool second)
 {
   const double pl = shup(pc), pr = shdn(pc);
-  const double s = second ? limited_slope(pc - pl, pr - pc, LIM) : 0.0;
+  const double s = second ? fast::slope_f(pc - pl, pr - pc, LIM) : 0.0;
   return fast::pratio_f(fma(0.5, shup(s), pl), fma(-0.5, s, pc));
 }
 
@@ -260,51 +263,72 @@ __device__ __forceinline__ Cons face_xie(const Prim& l, const Prim& r, int axis,
 {
   const double sensor = h * h * h;
   bool fb;
-  Cons f = fast::xie_core(l, r, axis, g, inv_gm1, sensor, fb, deg);
+  Cons f = fast::xie_core(l, r, axis, g, inv_gm1, sensor, fb);
+  deg = false;
   if (__any_sync(0xffffffffu, fb)) {
     if (fb) f = fast::xie_f(l, r, axis, g, inv_gm1, sensor, deg);
   }
   return f;
 }
 
-// RK = xie_am_hllc_p: the faces one at a time, each with its 5-face sensor.
-// The pressure ratios it needs come along the march: the y-faces' below and
-// above row j (carried, and this row's), and the x-faces' of rows j and j+1
-// (row j+1's from the pressure of the window's next row, carried on).
-template <int RK, int LIM, bool PAIR>
+// Advances the strip as march_strip does.  The x- and the y-face of a row are
+// evaluated back to back on the branch-free cores; faces those send back are
+// recomputed after one warp vote, their states rebuilt from the rings, so that
+// the common path keeps no face state alive for the repair.
+// RK = xie_am_hllc_p: each face with its 5-face sensor.  The pressure ratios
+// it needs come along the march: the y-faces' below and above row j (carried,
+// and this row's), and the x-faces' of rows j and j+1 (row j+1's from the
+// pressure of the window's next row, carried on).
+template <int RK, int LIM>
 __device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const double* __restrict__ u,
                                                    double* __restrict__ out, int c0, int j0, int H, double dt,
                                                    bool count_deg, MarchAcc& acc, StageRing& ring)
 {
+  constexpr bool XIE = RK == ECG_RIEMANN_XIE_AM_HLLC_P;
+  constexpr bool LM = RK == ECG_RIEMANN_LOWMACH_HLLC;
   const int lane = threadIdx.x & 31;
   const int x = c0 - 2 + lane;
   const int nx = P.g.nx, ny = P.g.ny;
   const double g = P.gamma, inv_gm1 = fast::frcp(g - 1.0);
-  const double idx = P.g.inv_dx, idy = P.g.inv_dy;
   const bool second = P.order > 1;
   const bool inner = lane >= 2 && lane < 2 + kCells;
   const bool cell_ok = inner && x < nx;
-  const bool xface = lane >= 2 && lane <= 2 + kCells;
-  const int xs = x < 0 ? 0 : (x < nx ? x : nx - 1);
   const int rhi = P.row_hi > 0 && P.row_hi < ny ? P.row_hi : ny;
   const int jend = j0 + H < rhi ? j0 + H : rhi;
   const int jlast = jend + 1;  // the last row the strip reads
+  const double dtx = dt * P.g.inv_dx, dty = dt * P.g.inv_dy;
 
   double* const col = &ring.v[0][0][lane];
+  double* const qcol = &ring.q[0][0][lane];
   const unsigned col_s = static_cast<unsigned>(__cvta_generic_to_shared(col));
+  const int left = lane > 0 ? -1 : 0, right = lane < 31 ? 1 : 0;  // neighbour columns (the end lanes' own)
   unsigned flips = 0;  // bit (row mod kRing): that staged row is a mirror image (my to negate)
-  // Strips whose 32 columns all lie in the domain take in-domain rows
-  // straight from the state, at a pointer that moves one row a request (the
-  // rows are requested in order); the ghost policy decides the rest.
-  const bool xin = c0 >= 2 && c0 + kLanes - 2 <= nx;
-  const long long pitch = P.g.pitch, pl = P.g.plane;
-  const double* rowp = u + static_cast<long long>(j0 - 2) * pitch + x;  // dereferenced only when in the domain
+  // Where this lane's column comes from in rows of the domain does not depend
+  // on the row (the state, a wrapped or clamped column of it, the ghost ring, a
+  // slab halo, or the constant state when null): found once, then a pointer
+  // that moves one row a request (the rows are requested in order).  Only the
+  // rows above and below the domain go through the ghost policy again; with
+  // the whole policy per cell, the strips on an x boundary ran 12 % longer than
+  // the others and held the launch up.
+  const CellSrc colsrc = cell_src(P, u, x, 0);
+  const long long cpl = colsrc.pl;
+  const long long cpitch = colsrc.p && ny > 1 ? cell_src(P, u, x, 1).p - colsrc.p : 0;
+  const long long pl = P.g.plane;
+  const double* rowp = colsrc.p + static_cast<long long>(j0 - 2) * cpitch;  // dereferenced only when in the domain
   // request row jr of this lane's column (an empty group past the strip's rows)
   auto put = [&](int jr) {
     if (jr <= jlast) {
       const int sl = jr & (kRing - 1);
-      const CellSrc c = xin && static_cast<unsigned>(jr) < static_cast<unsigned>(ny) ? CellSrc{rowp, pl, false}
-                                                                                     : cell_src(P, u, x, jr);
+      CellSrc c{rowp, cpl, false};
+      if (static_cast<unsigned>(jr) >= static_cast<unsigned>(ny)) {
+        if (P.bc.ring) {
+          c = cell_src(P, u, x, jr);
+        } else {
+          const int jj = ghost_row(P, jr, c.flip);
+          c.p = jj < 0 ? nullptr : colsrc.p + static_cast<long long>(jj) * cpitch;
+        }
+      }
+      if (!colsrc.p) c = CellSrc{nullptr, 0, false};
       flips = c.flip ? (flips | (1u << sl)) : (flips & ~(1u << sl));
       if (c.p) {
         const unsigned d = col_s + static_cast<unsigned>(sl * 4 * kLanes * 8);
@@ -320,36 +344,57 @@ __device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const d
         d[3 * kLanes] = P.bc.cst[3];
       }
     }
-    rowp += pitch;
+    rowp += cpitch;
     cp_async_commit();
   };
-  auto get = [&](int jr) {
-    const int sl = jr & (kRing - 1);
-    const double* d = col + sl * 4 * kLanes;
-    Cons c{d[0], d[kLanes], d[2 * kLanes], d[3 * kLanes]};
-    if ((flips >> sl) & 1u) c.my = -c.my;
-    return c;
+  auto conserved = [&](int jr) {
+    const double* d = col + (jr & (kRing - 1)) * 4 * kLanes;
+    return Cons{d[0], d[kLanes], d[2 * kLanes], d[3 * kLanes]};
+  };
+  // primitives of row jr of this lane's column, into the second ring
+  auto convert = [&](int jr) {
+    Cons c = conserved(jr);
+    if ((flips >> (jr & (kRing - 1))) & 1u) c.my = -c.my;
+    const Prim q = fast::to_prim_f(c, g);
+    double* d = qcol + (jr & (kPrim - 1)) * 3 * kLanes;
+    d[0] = q.u;
+    d[kLanes] = q.v;
+    d[2 * kLanes] = q.p;
+    return q;
+  };
+  // row jr of the column `dl` lanes over
+  auto prim = [&](int jr, int dl) {
+    const double* d = qcol + (jr & (kPrim - 1)) * 3 * kLanes + dl;
+    return Prim{col[(jr & (kRing - 1)) * 4 * kLanes + dl], d[0], d[kLanes], d[2 * kLanes]};
+  };
+  // The two states of the x-face on this lane's left in row j, and of the
+  // y-face above it, from the rings (the repair of a face).
+  auto xstates = [&](int j, Prim& l, Prim& r) {
+    const Prim a = prim(j, lane > 1 ? -2 : left), b = prim(j, left), c = prim(j, 0), d = prim(j, right);
+    l = plus_half(b, slope3<LIM>(a, b, c, second));
+    r = minus_half(c, slope3<LIM>(b, c, d, second));
+  };
+  auto ystates = [&](int j, Prim& l, Prim& r) {
+    const Prim a = prim(j - 1, 0), b = prim(j, 0), c = prim(j + 1, 0), d = prim(j + 2, 0);
+    l = plus_half(b, slope3<LIM>(a, b, c, second));
+    r = minus_half(c, slope3<LIM>(b, c, d, second));
   };
 
   // ---- prologue: stage rows j0-2 .. j0+1+kAhead; rows j0-2 .. j0+1 first ----
 #pragma unroll
   for (int r = -2; r <= 1 + kAhead; ++r) put(j0 + r);
   cp_async_wait<kAhead>();
-  Prim qa, qb, qc;  // rows j, j+1 and the slot of row j+2, by role
-  Prim s0, s1;      // y-slope of row j, and the slot of row j+1's
-  Cons g0, g1;      // y-face below row j, and the slot of the face above it
-  constexpr bool XIE = RK == ECG_RIEMANN_XIE_AM_HLLC_P;
+  Prim yp;  // row j's state at its upper y-face
+  Cons gb;  // the y-face below row j
   double yr_prev = 0.0, xr_cur = 0.0;  // XIE: pressure ratios of the y-face below row j, the x-face left of row j
   {
-    const Prim q_m2 = fast::to_prim_f(get(j0 - 2), g);
-    const Prim q_m1 = fast::to_prim_f(get(j0 - 1), g);
-    qa = fast::to_prim_f(get(j0), g);
-    qb = fast::to_prim_f(get(j0 + 1), g);
+    const Prim q_m2 = convert(j0 - 2), q_m1 = convert(j0 - 1), qa = convert(j0), qb = convert(j0 + 1);
     const Prim sy_m1 = slope3<LIM>(q_m2, q_m1, qa, second);
-    s0 = slope3<LIM>(q_m1, qa, qb, second);
+    const Prim s0 = slope3<LIM>(q_m1, qa, qb, second);
+    const Prim yl = plus_half(q_m1, sy_m1), yr = minus_half(qa, s0);
+    yp = plus_half(qa, s0);
     bool deg;
     if constexpr (XIE) {
-      const Prim yl = plus_half(q_m1, sy_m1), yr = minus_half(qa, s0);
       yr_prev = fast::pratio_f(yl.p, yr.p);
       const double xm1 = xface_ratio<LIM>(q_m1.p, second);
       xr_cur = xface_ratio<LIM>(qa.p, second);
@@ -358,117 +403,133 @@ __device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const d
       m = smin(m, shdn(xm1));
       m = smin(m, xr_cur);
       m = smin(m, shdn(xr_cur));
-      g0 = face_xie(yl, yr, 1, g, inv_gm1, clamp01(m), deg);
+      gb = face_xie(yl, yr, 1, g, inv_gm1, clamp01(m), deg);
     } else {
-      g0 = face_one<RK>(plus_half(q_m1, sy_m1), minus_half(qa, s0), 1, g, inv_gm1, deg);
+      gb = face_one<RK>(yl, yr, 1, g, inv_gm1, deg);
     }
     if (count_deg && deg && cell_ok && j0 < ny) acc.degenerate += 1;
   }
-  double* const obase = out + xs;
+  double* o = out + static_cast<long long>(j0) * P.g.pitch + (x < 0 ? 0 : (x < nx ? x : nx - 1));
   double rate_max = kLowest, rho_min = kMax, p_min = kMax;
 
-  // one row: row j's cells from rows j (q0), j+1 (q1) and the new row j+2
-  // (into q2), the y-slope of row j (sc; that of row j+1 into sn) and the
-  // y-face below row j (gb; the face above it into gt)
-  auto row = [&](int j, const Prim& q0, const Prim& q1, Prim& q2, const Prim& sc, Prim& sn, const Cons& gb, Cons& gt) {
+  for (int j = j0; j < jend; ++j) {
     put(j + 2 + kAhead);
     cp_async_wait<kAhead>();  // row j + 2 has landed
-    q2 = fast::to_prim_f(get(j + 2), g);
-    sn = slope3<LIM>(q0, q1, q2, second);
-    const Prim ql{shup(q0.rho), shup(q0.u), shup(q0.v), shup(q0.p)};
-    const Prim qr{shdn(q0.rho), shdn(q0.u), shdn(q0.v), shdn(q0.p)};
-    const Prim sx = slope3<LIM>(ql, q0, qr, second);
-    const Prim sxl{shup(sx.rho), shup(sx.u), shup(sx.v), shup(sx.p)};
-    Cons fl;
-    bool deg_x, deg_y, voted = true;
-    if constexpr (XIE) {
-      // sensors: the x-face on the left, from its own ratio and the y-faces'
-      // below and above cells i-1 and i; the y-face above, from its own ratio
-      // and the x-faces' left and right of cell i in rows j and j+1
-      const Prim xl = plus_half(ql, sxl), xrs = minus_half(q0, sx);
-      const Prim yl = plus_half(q0, sc), yrs = minus_half(q1, sn);
-      const double yr_cur = fast::pratio_f(yl.p, yrs.p);
-      const double xr_next = xface_ratio<LIM>(q1.p, second);
-      double my = yr_cur;
-      my = smin(my, xr_cur);
-      my = smin(my, shdn(xr_cur));
-      my = smin(my, xr_next);
-      my = smin(my, shdn(xr_next));
-      double mx = xr_cur;
-      mx = smin(mx, shup(yr_prev));
-      mx = smin(mx, shup(yr_cur));
-      mx = smin(mx, yr_prev);
-      mx = smin(mx, yr_cur);
-      gt = face_xie(yl, yrs, 1, g, inv_gm1, clamp01(my), deg_y);
-      fl = face_xie(xl, xrs, 0, g, inv_gm1, clamp01(mx), deg_x);
-      yr_prev = yr_cur;
-      xr_cur = xr_next;
-    } else if (PAIR) {
-      voted = face_pair<RK>(plus_half(ql, sxl), minus_half(q0, sx), plus_half(q0, sc), minus_half(q1, sn), g, inv_gm1,
-                            fl, gt, deg_x, deg_y);
-    } else {
-      gt = face_w<RK>(plus_half(q0, sc), minus_half(q1, sn), 1, g, inv_gm1, deg_y);
-      fl = face_w<RK>(plus_half(ql, sxl), minus_half(q0, sx), 0, g, inv_gm1, deg_x);
+    const Prim q2 = convert(j + 2);
+    __syncwarp();  // every lane's row j + 2 is in the rings
+    bool bx, by;
+    Cons gt, fl;
+    double mx = 0.0, my = 0.0;  // XIE: the sensors of the two faces
+    {
+      const Prim q1 = prim(j + 1, 0);
+      const Prim sn = slope3<LIM>(prim(j, 0), q1, q2, second);
+      const Prim yr = minus_half(q1, sn);
+      if constexpr (XIE) {
+        // sensors: the y-face above, from its own ratio and the x-faces' left
+        // and right of cell i in rows j and j+1; the x-face on the left, from
+        // its own ratio and the y-faces' below and above cells i-1 and i
+        const double yr_cur = fast::pratio_f(yp.p, yr.p);
+        const double xr_next = xface_ratio<LIM>(q1.p, second);
+        my = smin(smin(yr_cur, xr_cur), shdn(xr_cur));
+        my = smin(smin(my, xr_next), shdn(xr_next));
+        mx = smin(smin(xr_cur, shup(yr_prev)), shup(yr_cur));
+        mx = smin(smin(mx, yr_prev), yr_cur);
+        my = clamp01(my);
+        mx = clamp01(mx);
+        yr_prev = yr_cur;
+        xr_cur = xr_next;
+        gt = fast::xie_core(yp, yr, 1, g, inv_gm1, my * my * my, by);
+      } else if (RK == ECG_RIEMANN_RUSANOV) {
+        gt = fast::rusanov_core(yp, yr, 1, g, inv_gm1, by);
+      } else {
+        gt = fast::hllc_core<LM>(yp, yr, 1, g, inv_gm1, by);
+      }
+      yp = plus_half(q1, sn);
     }
+    {
+      const Prim q0 = prim(j, 0);
+      const Prim sx = slope3<LIM>(prim(j, left), q0, prim(j, right), second);
+      const Prim xp = plus_half(q0, sx), xr = minus_half(q0, sx);
+      const Prim xl{shup(xp.rho), shup(xp.u), shup(xp.v), shup(xp.p)};
+      if constexpr (XIE) fl = fast::xie_core(xl, xr, 0, g, inv_gm1, mx * mx * mx, bx);
+      else if (RK == ECG_RIEMANN_RUSANOV) fl = fast::rusanov_core(xl, xr, 0, g, inv_gm1, bx);
+      else fl = fast::hllc_core<LM>(xl, xr, 0, g, inv_gm1, bx);
+    }
+    if (__any_sync(0xffffffffu, bx || by)) {
+      Prim l, r;
+      bool deg_x = false, deg_y = false;
+      if (bx) {
+        xstates(j, l, r);
+        if constexpr (XIE) fl = fast::xie_f(l, r, 0, g, inv_gm1, mx * mx * mx, deg_x);
+        else fl = face_one<RK>(l, r, 0, g, inv_gm1, deg_x);
+      }
+      if (by) {
+        ystates(j, l, r);
+        if constexpr (XIE) gt = fast::xie_f(l, r, 1, g, inv_gm1, my * my * my, deg_y);
+        else gt = face_one<RK>(l, r, 1, g, inv_gm1, deg_y);
+      }
+      if (count_deg) {
+        // each face counts once per adjacent cell of this strip in the domain
+        // (count_hllc_degenerate_star_states, explicit_update.hpp:2-56); a
+        // face is degenerate only where the warp's fallback vote fired
+        const bool xface = lane >= 2 && lane <= 2 + kCells;
+        const bool left_ok = lane >= 3 && lane <= 2 + kCells && x - 1 < nx;
+        if (deg_x && xface) acc.degenerate += (left_ok ? 1 : 0) + (cell_ok ? 1 : 0);
+        if (deg_y && cell_ok) acc.degenerate += 1 + (j + 1 < jend ? 1 : 0);
+      }
+    }
+    // update (explicit_update.hpp:92-95) from the staged old state of row j, rounded
+    // once at its magnitude
     const Cons fr{shdn(fl.rho), shdn(fl.mx), shdn(fl.my), shdn(fl.E)};
-    if (count_deg && voted) {
-      // each face counts once per adjacent cell of this strip in the domain
-      // (count_hllc_degenerate_star_states, explicit_update.hpp:2-56); a
-      // face is degenerate only where the warp's fallback vote fired
-      const bool left_ok = lane >= 3 && lane <= 2 + kCells && x - 1 < nx;
-      if (deg_x && xface) acc.degenerate += (left_ok ? 1 : 0) + (cell_ok ? 1 : 0);
-      if (deg_y && cell_ok) acc.degenerate += 1 + (j + 1 < jend ? 1 : 0);
-    }
-    // update (explicit_update.hpp:92-95) from the staged old state of row j
-    const Cons old = get(j);
+    const Cons old = conserved(j);
     Cons n;
-    n.rho = old.rho - dt * ((fr.rho - fl.rho) * idx + (gt.rho - gb.rho) * idy);
-    n.mx = old.mx - dt * ((fr.mx - fl.mx) * idx + (gt.mx - gb.mx) * idy);
-    n.my = old.my - dt * ((fr.my - fl.my) * idx + (gt.my - gb.my) * idy);
-    n.E = old.E - dt * ((fr.E - fl.E) * idx + (gt.E - gb.E) * idy);
+    n.rho = old.rho - fma(dtx, fr.rho - fl.rho, dty * (gt.rho - gb.rho));
+    n.mx = old.mx - fma(dtx, fr.mx - fl.mx, dty * (gt.mx - gb.mx));
+    n.my = old.my - fma(dtx, fr.my - fl.my, dty * (gt.my - gb.my));
+    n.E = old.E - fma(dtx, fr.E - fl.E, dty * (gt.E - gb.E));
+    gb = gt;
     const Prim q = fast::to_prim_f(n, g);
     const double cs = fast::fsound_w(q.rho, q.p, g);
     if (cell_ok) {
-      double* o = obase + static_cast<long long>(j) * P.g.pitch;
       o[0] = n.rho;
       o[pl] = n.mx;
       o[2 * pl] = n.my;
       o[3 * pl] = n.E;
-      // running extrema as doubles (max/min skip a NaN operand, as the keys'
-      // NaN test does), turned into ordered keys once, after the strip
-      const double rate = (fabs(q.u) + cs) * idx + (fabs(q.v) + cs) * idy;
-      rate_max = fmax(rate_max, rate);
-      const bool bad = !isfinite(q.rho) || !isfinite(q.u) || !isfinite(q.v) || !isfinite(q.p) || !isfinite(n.E);
-      rho_min = fmin(rho_min, bad ? -kInf : q.rho);
-      p_min = fmin(p_min, bad ? -kInf : q.p);
-      acc.nonfinite += bad ? 1 : 0;
+      // running extrema as doubles: the comparisons skip a NaN as the keys'
+      // NaN test does, and a strip with a bad cell takes the floor at its end
+      const double rate = (fabs(q.u) + cs) * P.g.inv_dx + (fabs(q.v) + cs) * P.g.inv_dy;
+      rate_max = rate > rate_max ? rate : rate_max;
+      rho_min = q.rho < rho_min ? q.rho : rho_min;
+      p_min = q.p < p_min ? q.p : p_min;
+      // a nonfinite component (or velocity) makes the pressure nonfinite
+      if (!isfinite(q.p)) acc.nonfinite += 1;
     }
-  };
-
-  // (Six rows a trip, which hands the roles round by name with no register
-  // moves, measured 112.7 us against 75.8 us: the larger loop body costs
-  // more than the moves it saves.)
-  for (int j = j0; j < jend; ++j) {
-    row(j, qa, qb, qc, s0, s1, g0, g1);
-    qa = qb;
-    qb = qc;
-    s0 = s1;
-    g0 = g1;
+    o += P.g.pitch;
   }
   cp_async_wait<0>();  // no request outlives the strip
+  __syncwarp();        // nor a neighbour's read of this lane's rows the next strip's requests
+  if (acc.nonfinite > 0) rho_min = p_min = -kInf;
   acc.kmax = umax64(acc.kmax, okey(rate_max));
   acc.krho = umin64(acc.krho, okey(rho_min));
   acc.kp = umin64(acc.kp, okey(p_min));
 }
 
-// Registers: the register-loaded strips at most 128 a thread (4 blocks of 4
-// warps per SM), measured faster than the 166-register schedule the paired
-// faces get unbounded; the staged strips at most 168 (3 blocks), measured
-// faster than 128 for them (fewer registers spill).
+// Resident warps per SM the staged strips are compiled for.  They need 146 to
+// 150 registers unconstrained (the XIE flux 168 and some spill): 16 warps at 128
+// registers, without a spill, beat 12 for the HLLC fluxes on large grids
+// (2048x2048 132 against 137 us, 2560x640 equal), 20 at 96 registers spill and
+// lose (164 us, 70 us); the XIE flux (2560x640: 104 us at 12, 116 at 16) and
+// Rusanov, which spills at 128, stay at 12.
+template <int RK>
+constexpr int kStagedWarps = RK == ECG_RIEMANN_HLLC || RK == ECG_RIEMANN_LOWMACH_HLLC ? 16 : 12;
+
+// The register-loaded strips take at most 128 registers a thread (16 warps
+// per SM), measured faster than the 166-register schedule the paired faces get
+// unbounded.
 // STAGE: rows through the shared-memory ring (march_strip_staged), else
 // straight from global memory into registers (march_strip).
 template <int RK, int LIM, int WPB, bool PAIR, bool STAGE>
-__global__ void __launch_bounds__(WPB * 32, (STAGE ? 12 : 16) / WPB)
+__global__ void __launch_bounds__(WPB * 32, (STAGE ? kStagedWarps<RK> : 16) / WPB)
 fv_march_kernel(const EcgFvParams P, const double* __restrict__ u, double* __restrict__ out,
                 EcgStepStats* __restrict__ stats, const EcgDtCtl ctl, const int H)
 {
@@ -485,7 +546,7 @@ fv_march_kernel(const EcgFvParams P, const double* __restrict__ u, double* __res
   acc.init();
   if (c0 < P.g.nx) {
     if constexpr (STAGE)
-      march_strip_staged<RK, LIM, PAIR>(P, u, out, c0, j0, H, dt, ctl.count_degenerate != 0, acc,
+      march_strip_staged<RK, LIM>(P, u, out, c0, j0, H, dt, ctl.count_degenerate != 0, acc,
                                         ring[STAGE ? threadIdx.x >> 5 : 0]);
     else
       march_strip<RK, LIM, PAIR>(P, u, out, c0, j0, H, dt, ctl.count_degenerate != 0, acc);
@@ -493,20 +554,44 @@ fv_march_kernel(const EcgFvParams P, const double* __restrict__ u, double* __res
   block_commit<WPB * 32>(red, acc.kmax, acc.krho, acc.kp, acc.nonfinite, acc.degenerate, &stats[ctl.acc_slot]);
 }
 
-// Rows per warp: the given march_rows, else the smallest count that lets all
-// warp strips of the grid run in a single wave of resident warps (so no SM
-// idles in a tail), at least 8 so the per-strip prologue stays cheap.
+// Rows per warp: the count H with the least
+//   (H + 3) ((w + ceil w) / 2 + 0.15),   w = blocks(H) / resident blocks,
+// where 3 rows stand for a strip's prologue, and the mean of w and ceil w for
+// a last wave that is partly filled (its blocks run somewhat faster, and blocks
+// of the waves before it drift apart).  Fits the measured times of 15 grids
+// from 256x256 to 2048x2048 and H from 1 to 86 within 10 %; taking the rows
+// that give one wave of warps instead put 470 blocks on 444 slots at
+// 1021x509 (37 us a step, 27.5 with 12 rows) and ran 2048x2048 as a single
+// wave of 86 rows (219 us, 157 with 24).
+inline int rows_per_warp(int rows, int blocks_x, long long slots)
+{
+  int best = 1;
+  double least = 1.0e300;
+  for (int H = 1; H <= 96 && H <= rows; ++H) {
+    const double w = static_cast<double>(blocks_x) * ((rows + H - 1) / H) / static_cast<double>(slots);
+    const double c = (H + 3) * (0.5 * (w + ceil(w)) + 0.15);
+    if (c < least) {
+      least = c;
+      best = H;
+    }
+  }
+  return best;
+}
+
+// Two warps a block: the strips of a row of blocks overhang the grid by at
+// most one (four a block: 2 % to 8 % of the warps idle on odd widths).
 template <int RK, int LIM, bool PAIR, bool STAGE>
 cudaError_t launch_lim(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats, const EcgDtCtl& ctl,
                        cudaStream_t s)
 {
-  constexpr int WPB = 4;
+  constexpr int WPB = 2;
   const int strips = (p.g.nx + kCells - 1) / kCells;
   // a band of rows (the pipelined host step) or the whole grid
   const int rlo = p.row_hi > 0 ? p.row_lo : 0;
   const int rhi = p.row_hi > 0 && p.row_hi < p.g.ny ? p.row_hi : p.g.ny;
   const int rows = rhi - rlo;
   if (rows <= 0) return cudaSuccess;
+  const int bx = (strips + WPB - 1) / WPB;
   int H = p.march_rows;
   if (H <= 0) {
     static int blocks_per_sm = 0;
@@ -518,12 +603,9 @@ cudaError_t launch_lim(const EcgFvParams& p, const double* in, double* out, EcgS
         b = 1;
       blocks_per_sm = b;
     }
-    const long long slots = static_cast<long long>(p.sm_count > 0 ? p.sm_count : 148) * blocks_per_sm * WPB;
-    const long long per_col = slots / strips;  // warps available per strip column
-    H = per_col > 0 ? static_cast<int>((rows + per_col - 1) / per_col) : rows;
-    if (H < 8) H = 8;
+    H = rows_per_warp(rows, bx, static_cast<long long>(p.sm_count > 0 ? p.sm_count : 148) * blocks_per_sm);
   }
-  const dim3 grid((strips + WPB - 1) / WPB, (rows + H - 1) / H);
+  const dim3 grid(bx, (rows + H - 1) / H);
   fv_march_kernel<RK, LIM, WPB, PAIR, STAGE><<<grid, WPB * 32, 0, s>>>(p, in, out, stats, ctl, H);
   return cudaGetLastError();
 }

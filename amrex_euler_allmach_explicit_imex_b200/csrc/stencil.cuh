@@ -41,6 +41,23 @@ struct CellSrc {
   bool flip;
 };
 
+// The domain row behind row j outside the domain, -1 for the constant state;
+// flip: a wall's mirror image (my negated).
+__device__ __forceinline__ int ghost_row(const EcgFvParams& P, int j, bool& flip)
+{
+  const int ny = P.g.ny;
+  const bool low = j < 0;
+  const int policy = low ? P.bc.y_lo : P.bc.y_hi;
+  flip = policy == BC_REFLECT;
+  if (policy == BC_CONST) return -1;
+  if (policy == BC_PERIODIC) return wrapi(j, ny);
+  if (policy == BC_REFLECT) {  // row -1 - k mirrors row k, row ny + k mirrors row ny - 1 - k
+    const int r = low ? -j - 1 : 2 * ny - 1 - j;
+    return r < 0 ? 0 : (r > ny - 1 ? ny - 1 : r);
+  }
+  return low ? 0 : ny - 1;
+}
+
 __device__ __forceinline__ CellSrc cell_src(const EcgFvParams& P, const double* __restrict__ u, int i, int j)
 {
   const int nx = P.g.nx, ny = P.g.ny;
@@ -66,28 +83,9 @@ __device__ __forceinline__ CellSrc cell_src(const EcgFvParams& P, const double* 
     else i = P.bc.x_hi == BC_PERIODIC ? wrapi(i, nx) : nx - 1;
   }
   bool flip = false;
-  if (j < 0) {
-    if (P.bc.y_lo == BC_CONST) return CellSrc{nullptr, 0, false};
-    if (P.bc.y_lo == BC_PERIODIC) {
-      j = wrapi(j, ny);
-    } else if (P.bc.y_lo == BC_REFLECT) {
-      j = -j - 1;
-      j = j > ny - 1 ? ny - 1 : j;
-      flip = true;
-    } else {
-      j = 0;
-    }
-  } else if (j >= ny) {
-    if (P.bc.y_hi == BC_CONST) return CellSrc{nullptr, 0, false};
-    if (P.bc.y_hi == BC_PERIODIC) {
-      j = wrapi(j, ny);
-    } else if (P.bc.y_hi == BC_REFLECT) {
-      j = 2 * ny - 1 - j;  // row ny + k mirrors row ny - 1 - k
-      j = j < 0 ? 0 : j;
-      flip = true;
-    } else {
-      j = ny - 1;
-    }
+  if (j < 0 || j >= ny) {
+    j = ghost_row(P, j, flip);
+    if (j < 0) return CellSrc{nullptr, 0, false};
   }
   if (hs >= 0) {
     // the neighbour slab's cell, after the y policy (a corner ghost is the
@@ -489,10 +487,9 @@ cudaError_t launch_fv_step(const EcgFvParams& p, const double* in, double* out, 
 {
 #ifdef ECG_FAST_KERNEL
   // 0: column-strip kernel, x- and y-faces evaluated together, rows staged
-  // through shared memory by cp.async, 168 registers (default: 75.8 us at
-  // 2560x640); 3: the same with rows loaded into registers, 128 registers
-  // (77.8 us); 2: column-strip kernel, faces one after the other; 1:
-  // square-tile kernel
+  // through shared memory by cp.async (default: 57 us at 2560x640); 3: the
+  // same with rows loaded into registers (70 us); 2: column-strip kernel,
+  // faces one after the other; 1: square-tile kernel
   if (tile_y == 0) return march::launch(p, in, out, stats, ctl, s, true, true);
   if (tile_y == 3) return march::launch(p, in, out, stats, ctl, s, true, false);
   if (tile_y == 2) return march::launch(p, in, out, stats, ctl, s, false, false);
