@@ -5,14 +5,16 @@
 // (numerics/explicit_update.hpp:58-102) with dt held fixed, so
 //   gU0 = gU1 + (dq/dU)^T gq,   gq = sum over faces f of (dF_f/dq)^T gF_f,
 //   gF_{i+1/2} = dt/dx (gU1_{i+1} - gU1_i)   (and the same along y).
-// One thread per face evaluates the face's 4 x 16 Jacobian column by column
-// (forward-mode duals through the same limiter / Riemann branches the forward
-// takes, adjoint.cuh) and scatters (dF/dq)^T gF into the primitive gradients
-// of the four cells of its stencil, mapped through the boundary policy
-// (periodic images and outflow copies add to their source cell, the bubble
-// wall mirror flips the v component, constant inflow states receive nothing).
-// The scatter uses FP64 atomics, so the summation order and the last bits of
-// gU0 vary from run to run.  A second kernel applies (dq/dU)^T per cell.
+// One kernel does the whole transposed step on tiles of cells, gathering: it
+// stages the primitives and the cotangent of a tile and its halo in shared
+// memory, applies the transposed flux Jacobian of every face the tile's cells
+// depend on (reverse mode, adjoint.cuh), and every cell collects the
+// cotangents of its two faces and of the limited slopes it enters on each
+// axis.  Cells that ghost cells copy collect those ghosts' cotangents too (the
+// boundary policy transposed: outflow copies add to their source cell, the
+// bubble wall mirror flips the v component, constant inflow states receive
+// nothing; periodic axes wrap the tile instead).  No atomics: the result does
+// not vary from run to run.
 #include <cuda_runtime.h>
 
 #include <cstring>
@@ -23,10 +25,6 @@
 #include "adjoint.cuh"
 
 namespace {
-
-using ecg_adj::C4;
-using ecg_adj::Dual;
-using ecg_adj::P4;
 
 struct Src {
   int i, j;
@@ -76,110 +74,198 @@ __device__ Src source_of(const EcgFvParams& P, int i, int j)
   return s;
 }
 
-// Primitive state of (i, j), ghosts included (to_primitive, core/state_primitives.hpp:103-111).
-__device__ P4<double> prim_at(const EcgFvParams& P, const double* __restrict__ u, const Src& s)
-{
-  double rho, mx, my, E;
-  if (!s.valid) {
-    rho = P.bc.cst[0];
-    mx = P.bc.cst[1];
-    my = P.bc.cst[2];
-    E = P.bc.cst[3];
-  } else {
-    const long long o = static_cast<long long>(s.j) * P.g.pitch + s.i;
-    rho = u[o];
-    mx = u[o + P.g.plane];
-    my = u[o + 2 * P.g.plane];
-    E = u[o + 3 * P.g.plane];
-    if (s.flip) my = -my;
-  }
-  const double inv_rho = 1.0 / rho;
-  const double uu = mx * inv_rho, vv = my * inv_rho;
-  const double kin = 0.5 * rho * (uu * uu + vv * vv);
-  return P4<double>{rho, uu, vv, (P.gamma - 1.0) * (E - kin)};
-}
+// Tiles of at most TX x TY cells, of equal sizes up to one (so a tile on a wall
+// has both rows the wall mirrors, unless the grid has one row).  Staged per
+// tile: primitives of the cells within 3 of it (the faces one beyond its own
+// on each side and the slopes of their cells), cotangents within 2, and the
+// two state cotangents of each face -1 .. w+1 of its rows and -1 .. h+1 of its
+// columns.  632 faces over 320 threads: two a thread.
+//
+// Reverse mode costs about three flux evaluations a face where 16 forward
+// directional derivatives, one per primitive of the 4-cell stencil, cost some
+// thirty; with the gather in shared memory the 32 atomics a face and the
+// separate pass over the cells are gone too: one VJP at 256x256 325 us (158 +
+// 160 + 6 in three launches) -> 14.5 us (1024x1024: 178 us).
+constexpr int TX = 32, TY = 8, NT = 320;
+constexpr int PW = TX + 6, PH = TY + 6, PN = PW * PH;        // primitives, cells -3 .. T+2
+constexpr int GW = TX + 4, GH = TY + 4, GN = GW * GH;        // cotangents, cells -2 .. T+1
+constexpr int FXW = TX + 3, FYH = TY + 3;                    // faces -1 .. T+1
+constexpr int FX = FXW * TY, FY = TX * FYH, FN = FX + FY;
+constexpr size_t kSmem = sizeof(double) * (4 * PN + 4 * GN + 8 * FN);
 
-__device__ __forceinline__ double comp(const P4<double>& q, int m)
+template <int RK>
+__global__ void __launch_bounds__(NT, 2)
+step_vjp_kernel(const EcgFvParams P, const double* __restrict__ u0, const double* __restrict__ gu1, double dt,
+                double* __restrict__ gu0, int tiles_x, int tiles_y)
 {
-  return m == 0 ? q.rho : (m == 1 ? q.u : (m == 2 ? q.v : q.p));
-}
-
-// One thread per face of `axis`: gq of the face's 4-cell stencil += (dF/dq)^T gF.
-template <int AXIS>
-__global__ void face_vjp_kernel(const EcgFvParams P, const double* __restrict__ u0, const double* __restrict__ gu1,
-                                double dt, double* __restrict__ gq)
-{
+  extern __shared__ double sh[];
+  double* const prim = sh;           // 4 planes of PN: rho, u, v, p
+  double* const gu = prim + 4 * PN;  // 4 planes of GN
+  double* const gl = gu + 4 * GN;    // 4 planes of FN: cotangents of the faces' left / lower states
+  double* const gr = gl + 4 * FN;    // and of their right / upper states
   const int nx = P.g.nx, ny = P.g.ny;
-  const int fw = AXIS == 0 ? nx + 1 : nx;
-  const int fh = AXIS == 0 ? ny : ny + 1;
-  const long long nf = static_cast<long long>(fw) * fh;
   const long long n = static_cast<long long>(nx) * ny;
-  const double coef = dt * (AXIS == 0 ? P.g.inv_dx : P.g.inv_dy);
-  for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < nf;
-       e += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int fi = static_cast<int>(e % fw), fj = static_cast<int>(e / fw);
-    // cells L = c[1] (index f-1 along the axis) and R = c[2] (index f)
-    const int li = AXIS == 0 ? fi - 1 : fi, lj = AXIS == 0 ? fj : fj - 1;
-    const bool l_in = li >= 0 && lj >= 0;
-    const bool r_in = AXIS == 0 ? fi < nx : fj < ny;
-    double gF[4];
-    for (int m = 0; m < 4; ++m) {
-      const double gr = r_in ? gu1[static_cast<long long>(fj) * nx + fi + m * n] : 0.0;
-      const double gl = l_in ? gu1[static_cast<long long>(lj) * nx + li + m * n] : 0.0;
-      gF[m] = coef * (gr - gl);
-    }
-    if (gF[0] == 0.0 && gF[1] == 0.0 && gF[2] == 0.0 && gF[3] == 0.0) continue;
-    Src src[4];
-    P4<double> q[4];
-    for (int k = 0; k < 4; ++k) {
-      const int ci = AXIS == 0 ? fi - 2 + k : fi, cj = AXIS == 0 ? fj : fj - 2 + k;
-      src[k] = source_of(P, ci, cj);
-      q[k] = prim_at(P, u0, src[k]);
-    }
-    const int k0 = P.order > 1 ? 0 : 1, k1 = P.order > 1 ? 4 : 3;
-    for (int k = k0; k < k1; ++k) {
-      if (!src[k].valid) continue;
-      for (int m = 0; m < 4; ++m) {
-        P4<Dual> c[4];
-        for (int kk = 0; kk < 4; ++kk) {
-          c[kk] = P4<Dual>{Dual{q[kk].rho, 0.0}, Dual{q[kk].u, 0.0}, Dual{q[kk].v, 0.0}, Dual{q[kk].p, 0.0}};
-        }
-        Dual* slot = m == 0 ? &c[k].rho : (m == 1 ? &c[k].u : (m == 2 ? &c[k].v : &c[k].p));
-        slot->d = 1.0;
-        const C4<Dual> F = ecg_adj::t_face_flux(c, AXIS, P.gamma, P.riemann, P.order, P.limiter);
-        double g = gF[0] * F.rho.d + gF[1] * F.mx.d + gF[2] * F.my.d + gF[3] * F.E.d;
-        if (g == 0.0) continue;
-        if (src[k].flip && m == 2) g = -g;
-        atomicAdd(&gq[static_cast<long long>(src[k].j) * nx + src[k].i + m * n], g);
-      }
-    }
-  }
-}
+  const int bx = static_cast<int>(blockIdx.x) % tiles_x, by = static_cast<int>(blockIdx.x) / tiles_x;
+  auto cut = [](int cells, int k, int tiles) { return static_cast<int>(static_cast<long long>(cells) * k / tiles); };
+  const int i0 = cut(nx, bx, tiles_x), w = cut(nx, bx + 1, tiles_x) - i0;
+  const int j0 = cut(ny, by, tiles_y), h = cut(ny, by + 1, tiles_y) - j0;
+  const bool per_x = P.bc.x_lo == BC_PERIODIC, per_y = P.bc.y_lo == BC_PERIODIC;
+  const bool second = P.order > 1;
+  const double g = P.gamma, inv_gm1 = 1.0 / (g - 1.0);
+  const int tid = threadIdx.x;
 
-// gU0 = gU1 + (dq/dU)^T gq per cell.
-__global__ void cell_vjp_kernel(const EcgFvParams P, const double* __restrict__ u0, const double* __restrict__ gu1,
-                                const double* __restrict__ gq, double* __restrict__ gu0)
-{
-  const long long n = static_cast<long long>(P.g.nx) * P.g.ny;
-  const double gm1 = P.gamma - 1.0;
-  for (long long r = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; r < n;
-       r += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const double rho = u0[r], mx = u0[r + n], my = u0[r + 2 * n];
+  // ---- primitives (ghosts included: to_primitive, core/state_primitives.hpp:103-111) and cotangents ----
+  for (int e = tid; e < PN; e += NT) {
+    const int x = e % PW - 3, y = e / PW - 3;
+    const Src s = source_of(P, i0 + x, j0 + y);
+    double rho = P.bc.cst[0], mx = P.bc.cst[1], my = P.bc.cst[2], E = P.bc.cst[3];
+    if (s.valid) {
+      const long long o = static_cast<long long>(s.j) * nx + s.i;
+      rho = u0[o];
+      mx = u0[o + n];
+      my = s.flip ? -u0[o + 2 * n] : u0[o + 2 * n];
+      E = u0[o + 3 * n];
+    }
     const double inv_rho = 1.0 / rho;
     const double uu = mx * inv_rho, vv = my * inv_rho;
-    const double g0 = gq[r], g1 = gq[r + n], g2 = gq[r + 2 * n], g3 = gq[r + 3 * n];
-    gu0[r] = gu1[r] + g0 - (g1 * uu + g2 * vv) * inv_rho + g3 * gm1 * 0.5 * (uu * uu + vv * vv);
-    gu0[r + n] = gu1[r + n] + g1 * inv_rho - g3 * gm1 * uu;
-    gu0[r + 2 * n] = gu1[r + 2 * n] + g2 * inv_rho - g3 * gm1 * vv;
-    gu0[r + 3 * n] = gu1[r + 3 * n] + g3 * gm1;
+    prim[e] = rho;
+    prim[e + PN] = uu;
+    prim[e + 2 * PN] = vv;
+    prim[e + 3 * PN] = (g - 1.0) * (E - 0.5 * rho * (uu * uu + vv * vv));
+  }
+  for (int e = tid; e < GN; e += NT) {
+    int i = i0 + e % GW - 2, j = j0 + e / GW - 2;
+    if (per_x) i = wrapi(i, nx);
+    if (per_y) j = wrapi(j, ny);
+    const bool in = i >= 0 && i < nx && j >= 0 && j < ny;
+    const long long o = static_cast<long long>(j) * nx + i;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) gu[e + m * GN] = in ? gu1[o + m * n] : 0.0;
+  }
+  __syncthreads();
+
+  // ---- faces: cotangents of the two states of each ----
+  for (int e = tid; e < FN; e += NT) {
+    const bool xf = e < FX;
+    const int k = xf ? e : e - FX;
+    // the cell on the face's right / upper side, and the step to its neighbour
+    const int x = xf ? k % FXW - 1 : k % TX, y = xf ? k / FXW : k / TX - 1;
+    const bool used = xf ? (x <= w + 1 && y < h) : (x < w && y <= h + 1);
+    const int st = xf ? 1 : PW, gst = xf ? 1 : GW;
+    const int c = (y + 3) * PW + x + 3, gc = (y + 2) * GW + x + 2;
+    const double coef = dt * (xf ? P.g.inv_dx : P.g.inv_dy);
+    double wf[4];
+    bool any = false;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      wf[m] = used ? coef * (gu[gc + m * GN] - gu[gc - gst + m * GN]) : 0.0;
+      any = any || wf[m] != 0.0;
+    }
+    ecg_adj::State dl{0.0, 0.0, 0.0, 0.0}, dr{0.0, 0.0, 0.0, 0.0};
+    if (any) {
+      double ql[4], qr[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const double* q = prim + m * PN + c;
+        const double a = q[-2 * st], b = q[-st], d = q[0], f = q[st];
+        ql[m] = second ? b + 0.5 * ecg_adj::limited(b - a, d - b, P.limiter).s : b;
+        qr[m] = second ? d - 0.5 * ecg_adj::limited(d - b, f - d, P.limiter).s : d;
+      }
+      const ecg_adj::State l{ql[0], xf ? ql[1] : ql[2], xf ? ql[2] : ql[1], ql[3]};
+      const ecg_adj::State r{qr[0], xf ? qr[1] : qr[2], xf ? qr[2] : qr[1], qr[3]};
+      const ecg_adj::Flux wn{wf[0], xf ? wf[1] : wf[2], xf ? wf[2] : wf[1], wf[3]};
+      ecg_adj::reverse_face<RK>(l, r, g, inv_gm1, wn, dl, dr);
+    }
+    gl[e] = dl.rho;
+    gl[e + FN] = xf ? dl.un : dl.ut;
+    gl[e + 2 * FN] = xf ? dl.ut : dl.un;
+    gl[e + 3 * FN] = dl.p;
+    gr[e] = dr.rho;
+    gr[e + FN] = xf ? dr.un : dr.ut;
+    gr[e + 2 * FN] = xf ? dr.ut : dr.un;
+    gr[e + 3 * FN] = dr.p;
+  }
+  __syncthreads();
+
+  // ---- cells: gather the primitive cotangent, then (dq/dU)^T ----
+  for (int e = tid; e < TX * TY; e += NT) {
+    const int x = e % TX, y = e / TX;
+    if (x >= w || y >= h) continue;
+    const int c = (y + 3) * PW + x + 3;
+    double gq[4] = {0.0, 0.0, 0.0, 0.0};
+    // The cotangent of cell k of this cell's row (AXIS 0) or column, one axis'
+    // share: its two face states, and the slopes of cells k-1, k, k+1.  Faces
+    // outside -1 .. T+1 have no cotangent; a slope without one is not evaluated.
+    auto collect = [&](bool xa, int k, bool flip) {
+      const int fbase = xa ? y * FXW + 1 : FX + TX + x, fst = xa ? 1 : TX;
+      const int last = xa ? w + 1 : h + 1;
+      const int pbase = xa ? c - x : c - y * PW, pst = xa ? 1 : PW;
+      auto face = [&](const double* t, int f) { return f >= -1 && f <= last ? t[fbase + f * fst] : 0.0; };
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const double* L = gl + m * FN;
+        const double* R = gr + m * FN;
+        double v = face(L, k + 1) + face(R, k);
+        if (second) {
+          const double* q = prim + m * PN + pbase;
+#pragma unroll
+          for (int s = -1; s <= 1; ++s) {
+            const int kk = k + s;
+            const double gs = 0.5 * (face(L, kk + 1) - face(R, kk));
+            if (gs != 0.0) {
+              const double q0 = q[kk * pst];
+              const ecg_adj::Slope sl = ecg_adj::limited(q0 - q[(kk - 1) * pst], q[(kk + 1) * pst] - q0, P.limiter);
+              if (s == -1) v += gs * sl.db;
+              else if (s == 0) v += gs * (sl.da - sl.db);
+              else v -= gs * sl.da;
+            }
+          }
+        }
+        gq[m] += flip && m == 2 ? -v : v;
+      }
+    };
+    collect(true, x, false);
+    collect(false, y, false);
+    const int gi = i0 + x, gj = j0 + y;
+    if (!per_x) {
+      // ghost columns copy the edge column (a constant inflow none)
+      if (gi == 0 && P.bc.x_lo != BC_CONST) {
+        collect(true, -1, false);
+        collect(true, -2, false);
+      }
+      if (gi == nx - 1 && P.bc.x_hi != BC_CONST) {
+        collect(true, w, false);
+        collect(true, w + 1, false);
+      }
+    }
+    if (!per_y && (gj < 2 || gj >= ny - 2)) {
+      for (int t = 0; t < 4; ++t) {
+        const int ghost = t < 2 ? -1 - t : ny + t - 2;
+        const Src s = source_of(P, gi, ghost);
+        if (s.valid && s.j == gj) collect(false, ghost - j0, s.flip);
+      }
+    }
+    const double rho = prim[c], uu = prim[c + PN], vv = prim[c + 2 * PN];
+    const double inv_rho = 1.0 / rho, gm1 = g - 1.0;
+    const long long o = static_cast<long long>(gj) * nx + gi;
+    const double* gc = gu + (y + 2) * GW + x + 2;
+    gu0[o] = gc[0] + gq[0] - (gq[1] * uu + gq[2] * vv) * inv_rho + gq[3] * gm1 * 0.5 * (uu * uu + vv * vv);
+    gu0[o + n] = gc[GN] + gq[1] * inv_rho - gq[3] * gm1 * uu;
+    gu0[o + 2 * n] = gc[2 * GN] + gq[2] * inv_rho - gq[3] * gm1 * vv;
+    gu0[o + 3 * n] = gc[3 * GN] + gq[3] * gm1;
   }
 }
 
-int blocks_for(long long n, int nt)
+template <int RK>
+cudaError_t launch_vjp(const EcgFvParams& p, const double* u0, const double* gu1, double dt, double* gu0,
+                       cudaStream_t s)
 {
-  long long b = (n + nt - 1) / nt;
-  if (b > 148 * 16) b = 148 * 16;
-  return static_cast<int>(b < 1 ? 1 : b);
+  const cudaError_t e =
+      cudaFuncSetAttribute(step_vjp_kernel<RK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem));
+  if (e != cudaSuccess) return e;
+  const int tiles_x = (p.g.nx + TX - 1) / TX, tiles_y = (p.g.ny + TY - 1) / TY;
+  step_vjp_kernel<RK><<<tiles_x * tiles_y, NT, kSmem, s>>>(p, u0, gu1, dt, gu0, tiles_x, tiles_y);
+  return cudaGetLastError();
 }
 
 // Compact planes (i fastest, no padding) of the context's grid.
@@ -191,12 +277,19 @@ EcgFvParams compact_params(ecg_ctx* c)
   return p;
 }
 
-bool ensure_adj(ecg_ctx* c)
+// The record the forward step reduces into; nothing reads it, so it is
+// initialised once and left to accumulate.
+bool ensure_stats(ecg_ctx* c)
 {
-  if (c->adj_gq) return true;
-  const size_t n = static_cast<size_t>(c->grid.nx) * c->grid.ny;
-  return ecgi::cuda_ok(c, cudaMalloc(&c->adj_gq, sizeof(double) * 4 * n), "alloc adjoint") &&
-         ecgi::cuda_ok(c, cudaMalloc(&c->adj_stats, sizeof(EcgStepStats)), "alloc adjoint stats");
+  if (c->adj_stats) return true;
+  return ecgi::cuda_ok(c, cudaMalloc(&c->adj_stats, sizeof(EcgStepStats)), "alloc adjoint stats") &&
+         ecgi::cuda_ok(c, c->ops->init_stats(c->adj_stats, 1, 0.0, c->stream), "init stats");
+}
+
+// Whether two arrays of n doubles share a byte.
+bool overlap(const double* a, const double* b, long long n)
+{
+  return a < b + n && b < a + n;
 }
 
 }  // namespace
@@ -211,7 +304,7 @@ ecg_status ecg_explicit_step_device(ecg_ctx* c, const double* u0, double dt, dou
     c->err = "exact-Dirichlet ghost rings are not supported on caller arrays";
     return ECG_ERR_UNSUPPORTED;
   }
-  if (!ensure_adj(c)) return ECG_ERR_CUDA;
+  if (!ensure_stats(c)) return ECG_ERR_CUDA;
   EcgDtCtl ctl;
   std::memset(&ctl, 0, sizeof(ctl));
   ctl.dt = dt;
@@ -219,7 +312,6 @@ ecg_status ecg_explicit_step_device(ecg_ctx* c, const double* u0, double dt, dou
   ctl.read_slot = 0;
   ctl.acc_slot = 0;
   ctl.reset_slot = -1;
-  if (!ecgi::cuda_ok(c, c->ops->init_stats(c->adj_stats, 1, 0.0, c->stream), "init stats")) return ECG_ERR_CUDA;
   if (!ecgi::cuda_ok(c, c->ops->fv_step(p, u0, u1, c->adj_stats, ctl, c->tile_y, c->stream), "fv_step"))
     return ECG_ERR_CUDA;
   return ECG_OK;
@@ -237,17 +329,24 @@ ecg_status ecg_explicit_step_vjp_device(ecg_ctx* c, const double* u0, double dt,
     c->err = "the adjoint covers rusanov, hllc and lowmach_hllc";
     return ECG_ERR_UNSUPPORTED;
   }
-  if (!ensure_adj(c)) return ECG_ERR_CUDA;
-  const long long n = static_cast<long long>(c->grid.nx) * c->grid.ny;
-  if (!ecgi::cuda_ok(c, cudaMemsetAsync(c->adj_gq, 0, sizeof(double) * 4 * n, c->stream), "memset")) return ECG_ERR_CUDA;
-  const long long nfx = static_cast<long long>(c->grid.nx + 1) * c->grid.ny;
-  const long long nfy = static_cast<long long>(c->grid.nx) * (c->grid.ny + 1);
-  face_vjp_kernel<0><<<blocks_for(nfx, 128), 128, 0, c->stream>>>(p, u0, g_u1, dt, c->adj_gq);
-  if (!ecgi::cuda_ok(c, cudaGetLastError(), "face vjp x")) return ECG_ERR_CUDA;
-  face_vjp_kernel<1><<<blocks_for(nfy, 128), 128, 0, c->stream>>>(p, u0, g_u1, dt, c->adj_gq);
-  if (!ecgi::cuda_ok(c, cudaGetLastError(), "face vjp y")) return ECG_ERR_CUDA;
-  cell_vjp_kernel<<<blocks_for(n, 256), 256, 0, c->stream>>>(p, u0, g_u1, c->adj_gq, g_u0);
-  if (!ecgi::cuda_ok(c, cudaGetLastError(), "cell vjp")) return ECG_ERR_CUDA;
+  const long long n = 4LL * c->grid.nx * c->grid.ny;
+  // Tiles read u0 and g_u1 around the cells other tiles write: a result that
+  // lies on either of them goes through the context's scratch.
+  const bool scratch = overlap(g_u0, u0, n) || overlap(g_u0, g_u1, n);
+  if (scratch && !c->adj_gq &&
+      !ecgi::cuda_ok(c, cudaMalloc(&c->adj_gq, sizeof(double) * n), "alloc adjoint"))
+    return ECG_ERR_CUDA;
+  double* out = scratch ? c->adj_gq : g_u0;
+  cudaError_t e;
+  switch (c->cfg.riemann) {
+    case ECG_RIEMANN_RUSANOV: e = launch_vjp<ECG_RIEMANN_RUSANOV>(p, u0, g_u1, dt, out, c->stream); break;
+    case ECG_RIEMANN_LOWMACH_HLLC: e = launch_vjp<ECG_RIEMANN_LOWMACH_HLLC>(p, u0, g_u1, dt, out, c->stream); break;
+    default: e = launch_vjp<ECG_RIEMANN_HLLC>(p, u0, g_u1, dt, out, c->stream); break;
+  }
+  if (!ecgi::cuda_ok(c, e, "step vjp")) return ECG_ERR_CUDA;
+  if (scratch && !ecgi::cuda_ok(c, cudaMemcpyAsync(g_u0, out, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream),
+                                "copy vjp"))
+    return ECG_ERR_CUDA;
   return ECG_OK;
 }
 

@@ -565,9 +565,10 @@ fv_march_kernel(const EcgFvParams P, const double* __restrict__ u, double* __res
 // wave of 86 rows (219 us, 157 with 24).
 inline int rows_per_warp(int rows, int blocks_x, long long slots)
 {
-  int best = 1;
+  const int lo = (rows + 65534) / 65535;  // blocks along y
+  int best = lo;
   double least = 1.0e300;
-  for (int H = 1; H <= 96 && H <= rows; ++H) {
+  for (int H = lo; H <= 96 && H <= rows; ++H) {
     const double w = static_cast<double>(blocks_x) * ((rows + H - 1) / H) / static_cast<double>(slots);
     const double c = (H + 3) * (0.5 * (w + ceil(w)) + 0.15);
     if (c < least) {
