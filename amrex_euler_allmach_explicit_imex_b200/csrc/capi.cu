@@ -174,6 +174,7 @@ EcgProblem problem_of(ecg_ctx* c, bool imex_policy)
   EcgBc bc;
   EcgProblem pr;
   make_bc(c->cfg, imex_policy, bc, pr);
+  pr.star = c->d_star;
   return pr;
 }
 
@@ -245,6 +246,7 @@ ecg_ctx::~ecg_ctx()
   cudaFree(d_ring);
   cudaFree(d_stats);
   cudaFree(d_state_stats);
+  cudaFree(d_star);
   cudaFree(adj_gq);
   cudaFree(adj_stats);
   cudaFreeHost(h_stats);
@@ -417,6 +419,13 @@ ecg_status ecg_create(ecg_ctx** out, const ecg_run_config* cfg, const ecg_gpu_op
   ok = ok && cuda_ok(c, cudaMallocHost(&c->h_stats, sizeof(EcgStepStats) * c->stats_cap), "alloc host stats");
   ok = ok && cuda_ok(c, cudaMalloc(&c->d_state_stats, sizeof(EcgStateStats)), "alloc state stats");
   ok = ok && cuda_ok(c, cudaMallocHost(&c->h_state_stats, sizeof(EcgStateStats)), "alloc host state stats");
+  // the exact ghosts of a Toro problem sample one Riemann solution: its star
+  // state is part of the configuration
+  const EcgProblem pr = problem_of(c, false);
+  if (pr.ring_kind == RING_TORO) {
+    ok = ok && cuda_ok(c, cudaMalloc(&c->d_star, sizeof(double) * 2), "alloc star");
+    ok = ok && cuda_ok(c, c->ops->riemann_star(pr, c->d_star, c->stream), "riemann star");
+  }
   ok = ok && cuda_ok(c, cudaStreamSynchronize(c->stream), "sync");
   if (!ok) {
     std::fprintf(stderr, "ecg_create: %s\n", c->err.c_str());

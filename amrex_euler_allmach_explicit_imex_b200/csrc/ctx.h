@@ -73,6 +73,7 @@ struct ecg_ctx {
   bool slab() const { return halo_lo || halo_hi; }
   EcgImexState* imex = nullptr;
   EcgOutput* out = nullptr;  // output writers' buffers (output.cu)
+  double* d_star = nullptr;  // star state of a Toro problem with exact ghosts (EcgProblem::star)
   // adjoint workspace (adjoint.cu): a result that overlaps an input, one stats record
   double* adj_gq = nullptr;
   EcgStepStats* adj_stats = nullptr;

@@ -40,6 +40,7 @@ struct EcgProblem {
   int problem;
   double gamma;
   double toro_l[4], toro_r[4];  // primitive rho,u,v,p
+  const double* star;  // device: pressure and velocity of their star state, or null (solved where it is needed)
   double interface_x, interface_y;
   double vortex_cx, vortex_cy, density_outer, density_inner, pressure, mach;
   double blob_cx, blob_cy, blob_radius, velocity_x, velocity_y;
@@ -158,6 +159,7 @@ struct EcgStencilOps {
   cudaError_t (*init_state_stats)(EcgStateStats* st, cudaStream_t s);
   cudaError_t (*seed_stats)(EcgStepStats* stats, const EcgStateStats* st, cudaStream_t s);
   cudaError_t (*init_state)(const EcgFvParams& p, const EcgProblem& pr, double* u, cudaStream_t s);
+  cudaError_t (*riemann_star)(const EcgProblem& pr, double* out, cudaStream_t s);
 };
 
 namespace ecg_fast {

@@ -53,9 +53,13 @@ __device__ void pressure_fn(double p, const Prim& q, double g, double& f, double
   d = 1.0 / (q.rho * a) * pow(ratio, -(g + 1.0) / (2.0 * g));
 }
 
-__device__ Prim riemann_sample(double x, double t, const Prim& l, const Prim& r, double g, double x0)
+// Pressure and velocity between the two nonlinear waves: they depend on the
+// two states alone.
+struct RiemannStar {
+  double p, u;
+};
+__device__ RiemannStar riemann_star(const Prim& l, const Prim& r, double g)
 {
-  if (t <= 0.0) return x < x0 ? l : r;
   const double al = sqrt(g * l.p / l.rho), ar = sqrt(g * r.p / r.rho);
   double p = smax(1.0e-12, 0.5 * (l.p + r.p) - 0.125 * (r.u - l.u) * (l.rho + r.rho) * (al + ar));
   for (int it = 0; it < 80; ++it) {
@@ -74,7 +78,16 @@ __device__ Prim riemann_sample(double x, double t, const Prim& l, const Prim& r,
   double fl, dl, fr, dr;
   pressure_fn(p, l, g, fl, dl);
   pressure_fn(p, r, g, fr, dr);
-  const double ps = p, us = 0.5 * (l.u + r.u + fr - fl);
+  return RiemannStar{p, 0.5 * (l.u + r.u + fr - fl)};
+}
+
+// The solution at (x, t), the star state known.
+__device__ Prim riemann_sample(double x, double t, const Prim& l, const Prim& r, double g, double x0,
+                               const RiemannStar& star)
+{
+  if (t <= 0.0) return x < x0 ? l : r;
+  const double al = sqrt(g * l.p / l.rho), ar = sqrt(g * r.p / r.rho);
+  const double ps = star.p, us = star.u;
   const double xi = (x - x0) / t;
   const double gm1 = g - 1.0, gp1 = g + 1.0;
   if (xi <= us) {
@@ -107,6 +120,12 @@ __device__ Prim riemann_sample(double x, double t, const Prim& l, const Prim& r,
   const double uu = 2.0 / gp1 * (-ar + 0.5 * gm1 * r.u + xi);
   const double a = 2.0 / gp1 * (ar - 0.5 * gm1 * (r.u - xi));
   return Prim{r.rho * pow(a / ar, 2.0 / gm1), uu, r.v, r.p * pow(a / ar, 2.0 * g / gm1)};
+}
+
+__device__ Prim riemann_sample(double x, double t, const Prim& l, const Prim& r, double g, double x0)
+{
+  if (t <= 0.0) return x < x0 ? l : r;
+  return riemann_sample(x, t, l, r, g, x0, riemann_star(l, r, g));
 }
 
 // periodic_nearest_delta, problems/problem_state_functions.hpp:32-43
