@@ -68,7 +68,7 @@ struct GmresArgs {
   double* r;     // n: residual recurrence
   float* V32;    // (m+1) x n (mixed)
   double* part;  // residual_kernel: 2 x its blocks
-  double* acc;   // three accumulator rows of ld doubles, zeroed by the host before the launch
+  double* acc;   // three accumulator rows of ld entries, zeroed by the host before the launch
   double* dpt;   // deterministic mode: three tables of per-block partial sums (nblocks x ld each)
   double* R;     // column-major (m+1) x m
   GridBar* bar;
@@ -84,6 +84,7 @@ struct GmresArgs {
   int reorth;         // mixed: DGKS test of the FP32-basis cycles, 1 as the FP64 solve, 0 severe cancellation only
   int kres;           // basis vectors resident in shared memory on each block's rows
   int prow;           // rows of a block (the last may have fewer)
+  int wrows;          // rows of w kept in shared memory (prow, or 0: in global memory)
   int det;            // grid sums in a fixed order (bit-reproducible solves)
   long long spin_limit;
   // Chained solves (gmres_enqueue): gate[0] is set once a phase of the chain
@@ -352,11 +353,12 @@ struct Smem {
   double* coef;
   double* wpart;
   double* scratch;
+  double* ws;  // w on the block's rows (when it fits)
   double* vs;  // resident basis vectors (TV)
   double* dpart;
   double* cnt;  // block 0: vector accesses per row of the solve, [0] FP64 vectors, [1] basis vectors stored as FP32
 };
-__device__ __forceinline__ Smem carve(double* base, int m)
+__device__ __forceinline__ Smem carve(double* base, int m, int wrows = 0)
 {
   const int L = m + 8;
   Smem s;
@@ -370,7 +372,8 @@ __device__ __forceinline__ Smem carve(double* base, int m)
   s.scratch = s.wpart + NW;
   s.cnt = s.scratch + NT + L;
   s.dpart = s.cnt + 2;
-  s.vs = s.dpart + NW * dots_ld(m);
+  s.ws = s.dpart + NW * dots_ld(m);
+  s.vs = s.ws + wrows;
   return s;
 }
 // bytes of the fixed part; the resident basis vectors follow it
@@ -415,35 +418,51 @@ __device__ __forceinline__ void warp_partial(double v, double* wpart)
 // writes its partials last adds them up in block order into the row before
 // the grid barrier (acc_settle), so every launch on the same inputs gives the
 // same bits.  Maxima are exact in any order and stay atomic.
+//
+//
+// Where every warp adds the sums it has (the small-block dot products), an
+// entry sits in a 128-byte line of its own (stride kAccLine): packed together,
+// some 60 entries from 148 blocks queue on four L2 lines (256x256 FP64: 22.5 us
+// an iteration, 18.8 apart).  Large blocks add a warp's 32 neighbouring entries
+// with one instruction, which packed entries serve best (512x512: 64.3 us an
+// iteration packed, 65.9 apart).
+constexpr int kAccLine = 16;
+constexpr int kSmallRows = 512;  // rows a block may have in the small-block layouts
+__host__ __device__ constexpr int acc_stride(int prow) { return prow <= kSmallRows ? kAccLine : 1; }
 struct Acc {
   double* rows;
   int ld;
+  int stride;   // doubles between the entries of a row
   double* dpt;  // per-block partial tables (deterministic mode), else null
-  __device__ __forceinline__ double* row(unsigned int k) const { return rows + (k % 3) * ld; }
+  __device__ __forceinline__ double* row(unsigned int k) const
+  {
+    return rows + static_cast<size_t>(k % 3) * ld * stride;
+  }
 };
 
 // Destination of one block's partial sums of one reduction.
 struct SumSink {
   double* p;
-  bool det;
+  int stride;  // of the row's entries; 0: the block's own slot (deterministic mode)
 };
 __device__ __forceinline__ SumSink sink(const Acc& A, unsigned int k)
 {
-  if (A.dpt) return SumSink{A.dpt + (static_cast<size_t>(k % 3) * gridDim.x + blockIdx.x) * A.ld, true};
-  return SumSink{A.row(k), false};
+  if (A.dpt) return SumSink{A.dpt + (static_cast<size_t>(k % 3) * gridDim.x + blockIdx.x) * A.ld, 0};
+  return SumSink{A.row(k), A.stride};
 }
 
 __device__ __forceinline__ void acc_add(const SumSink& s, int q, double v)
 {
-  if (s.det) s.p[q] = v;
-  else atomicAdd(s.p + q, v);
+  if (s.stride == 0) s.p[q] = v;
+  else atomicAdd(s.p + q * s.stride, v);
 }
 
 // Maxima are nonnegative or NaN (with the sign bit clear), which order as
 // their bit patterns, NaN above every number.
-__device__ __forceinline__ void acc_max(double* row, int q, double v)
+__device__ __forceinline__ void acc_max(const Acc& A, unsigned int k, int q, double v)
 {
-  atomicMax(reinterpret_cast<unsigned long long*>(row + q), static_cast<unsigned long long>(__double_as_longlong(v)));
+  atomicMax(reinterpret_cast<unsigned long long*>(A.row(k) + q * A.stride),
+            static_cast<unsigned long long>(__double_as_longlong(v)));
 }
 
 // Deterministic mode, after every block has written its partial sums of
@@ -473,7 +492,7 @@ __device__ __forceinline__ void acc_settle(const Acc& A, GridBar* bar, unsigned 
     for (int b = lane; b < static_cast<int>(gridDim.x); b += 32) s += __ldcg(tab + static_cast<size_t>(b) * A.ld + q);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) __stcg(row + q, s);
+    if (lane == 0) __stcg(row + q * A.stride, s);
   }
   __syncthreads();
 }
@@ -483,10 +502,10 @@ __device__ __forceinline__ void acc_settle(const Acc& A, GridBar* bar, unsigned 
 __device__ __forceinline__ void acc_read(const Acc& A, unsigned int& k, int ne, double* out)
 {
   const double* r = A.row(k);
-  for (int q = threadIdx.x; q < ne; q += NT) out[q] = __ldcg(r + q);
+  for (int q = threadIdx.x; q < ne; q += NT) out[q] = __ldcg(r + q * A.stride);
   if (blockIdx.x == 0) {
     double* z = A.row(k + 2);
-    for (int q = threadIdx.x; q < A.ld; q += NT) z[q] = 0.0;
+    for (int q = threadIdx.x; q < A.ld; q += NT) z[q * A.stride] = 0.0;
   }
   ++k;
   __syncthreads();
@@ -592,7 +611,7 @@ __device__ __forceinline__ double warp_reduce_scatter(double (&s)[DG], int lane)
 // count of w to entry nvec + 1.  Every thread takes part: DG sums a pass over its rows
 // (w read once a pass), a reduce-scatter of the DG sums in each warp, then
 // the warps' partials summed in warp order.
-template <typename TV>
+template <typename TV, bool RES>
 __device__ __forceinline__ void block_dots(const Basis<TV>& bs, const double* __restrict__ w, Rows rw, int nvec,
                                            bool with_norm, const SumSink& row, double* dpart, bool pair)
 {
@@ -603,7 +622,8 @@ __device__ __forceinline__ void block_dots(const Basis<TV>& bs, const double* __
   __syncthreads();  // w of the block's rows is complete
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tot = nvec + (with_norm ? 2 : 0);
-  if (rw.r1 - rw.r0 <= 32 * SMALL) {
+  static_assert(32 * SMALL == kSmallRows, "");
+  if (bs.P <= kSmallRows) {
     // Few rows (an L2-resident system): warp k takes vectors k, k + NW, ...
     // over all the block's rows, lanes striding the rows with w in registers;
     // one round trip a vector and no block-wide step between vectors.
@@ -613,32 +633,61 @@ __device__ __forceinline__ void block_dots(const Basis<TV>& bs, const double* __
       const int q = rw.r0 + lane + 32 * k;
       wr[k] = q < rw.r1 ? w[q] : 0.0;
     }
-    for (int i = warp; i < tot; i += NW) {
-      double sm = 0.0;
-      if (i < nvec) {
-        TV av[SMALL];
-        if (i < bs.K) {
-          const TV* pv = bs.s + i * bs.P + lane;
+    // Two vectors a pass (warp, warp + NW): two independent sums hide
+    // each other's FMA latency and share one reduce-scatter of the warp (with
+    // the accumulators apart: 256x256 FP64 22.6 -> 18.8 us an iteration).
+    // (One at a time without resident vectors: a basis too long for them.)
+    constexpr int G = RES ? 2 : 1;
+    for (int i0 = warp; i0 < tot; i0 += G * NW) {
+      double sm[G];
 #pragma unroll
-          for (int k = 0; k < SMALL; ++k) av[k] = rw.r0 + lane + 32 * k < rw.r1 ? pv[32 * k] : TV(0);
-        } else {
-          const TV* pv = V + static_cast<long long>(i) * n + rw.r0 + lane;  // rows at immediate offsets
+      for (int v = 0; v < G; ++v) sm[v] = 0.0;
+      if (i0 + (G - 1) * NW < bs.K) {  // all resident
+        const TV* pv = bs.s + i0 * bs.P + lane;
+        const int step = NW * bs.P;
 #pragma unroll
-          for (int k = 0; k < SMALL; ++k) av[k] = rw.r0 + lane + 32 * k < rw.r1 ? __ldcg(pv + 32 * k) : TV(0);
+        for (int k = 0; k < SMALL; ++k) {
+          const bool in = rw.r0 + lane + 32 * k < rw.r1;
+#pragma unroll
+          for (int v = 0; v < G; ++v) {
+            const double a = in && i0 + v * NW < nvec ? static_cast<double>(pv[v * step + 32 * k]) : 0.0;
+            sm[v] += a * wr[k];
+          }
         }
-#pragma unroll
-        for (int k = 0; k < SMALL; ++k) sm += static_cast<double>(av[k]) * wr[k];
-      } else if (i == nvec) {
-#pragma unroll
-        for (int k = 0; k < SMALL; ++k) sm += wr[k] * wr[k];
       } else {
 #pragma unroll
-        for (int k = 0; k < SMALL; ++k)
-          if (!isfinite(wr[k])) sm = 1.0;
+        for (int v = 0; v < G; ++v) {
+          const int i = i0 + v * NW;
+          if (i >= nvec) break;
+          TV av[SMALL];
+          if (i < bs.K) {
+            const TV* pv = bs.s + i * bs.P + lane;
+#pragma unroll
+            for (int k = 0; k < SMALL; ++k) av[k] = rw.r0 + lane + 32 * k < rw.r1 ? pv[32 * k] : TV(0);
+          } else {
+            const TV* pv = V + static_cast<long long>(i) * n + rw.r0 + lane;  // rows at immediate offsets
+#pragma unroll
+            for (int k = 0; k < SMALL; ++k) av[k] = rw.r0 + lane + 32 * k < rw.r1 ? __ldcg(pv + 32 * k) : TV(0);
+          }
+#pragma unroll
+          for (int k = 0; k < SMALL; ++k) sm[v] += static_cast<double>(av[k]) * wr[k];
+        }
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
-      if (lane == 0) acc_add(row, i, sm);
+      for (int v = 0; v < G; ++v) {
+        const int i = i0 + v * NW;
+        if (i == nvec) {
+#pragma unroll
+          for (int k = 0; k < SMALL; ++k) sm[v] += wr[k] * wr[k];
+        } else if (i == nvec + 1) {
+#pragma unroll
+          for (int k = 0; k < SMALL; ++k)
+            if (!isfinite(wr[k])) sm[v] = 1.0;
+        }
+      }
+      const double t = warp_reduce_scatter<G>(sm, lane);  // lane (32 / G) v holds sum v
+      const int i = i0 + lane / (32 / G) * NW;
+      if ((lane & (32 / G - 1)) == 0 && i < tot) acc_add(row, i, t);
     }
     __syncthreads();
     return;
@@ -903,8 +952,7 @@ __device__ __forceinline__ double sweep_next(Rows rw, const Basis<TV>& bs, const
 // of x0 by any other row.
 template <typename TV, bool RES>
 __device__ SolveState krylov(const GmresArgs& a, const double* __restrict__ bvec, const double* x0vec, double* xvec,
-                             TV* __restrict__ V, double* __restrict__ w,
-                             double* __restrict__ rres, int kmax, double tol, double restart_rtol, int reorth,
+                             TV* __restrict__ V, double* __restrict__ rres, int kmax, double tol, double restart_rtol, int reorth,
                              unsigned int& gen, unsigned int& nred, unsigned int& nset, double* shbase)
 {
   const long long n = a.n;
@@ -912,11 +960,15 @@ __device__ SolveState krylov(const GmresArgs& a, const double* __restrict__ bvec
   const bool wide = rw.r1 - rw.r0 > NT;  // two rows a thread per pass
   // FP32 basis of an even-sized system: adjacent row pairs, 8-byte loads
   const bool pair = sizeof(TV) == 4 && wide && (n & 1) == 0;
-  const Smem S = carve(shbase, a.m);
+  const Smem S = carve(shbase, a.m, a.wrows);
+  // w has no reader outside its block: a large block keeps it in shared memory
+  // when it fits (never beside a resident basis, whose instantiation leaves the
+  // choice out for its registers)
+  double* const w = !RES && a.wrows ? S.ws - rw.r0 : a.w;
   // RES = false: no resident vectors (K a constant 0, the shared-memory
   // paths compiled out, the register budget of the plain solve)
   const Basis<TV> bs{V, n, reinterpret_cast<TV*>(S.vs), RES ? a.kres : 0, a.prow, rw.r0};
-  const Acc A{a.acc, a.ld, a.det ? a.dpt : nullptr};
+  const Acc A{a.acc, a.ld, acc_stride(a.prow), a.det ? a.dpt : nullptr};
   SolveState st;
   st.it = 0;
   st.best_it = 0;
@@ -936,8 +988,8 @@ __device__ SolveState krylov(const GmresArgs& a, const double* __restrict__ bvec
     bmax = block_max(bmax, S.scratch);
     rmax = block_max(rmax, S.scratch);
     if (threadIdx.x == 0) {
-      acc_max(A.row(nred), 1, bmax);
-      acc_max(A.row(nred), 2, rmax);
+      acc_max(A, nred, 1, bmax);
+      acc_max(A, nred, 2, rmax);
     }
     acc_settle(A, a.bar, nred, 1, nset);
   }
@@ -1037,7 +1089,7 @@ __device__ SolveState krylov(const GmresArgs& a, const double* __restrict__ bvec
     if (!fused) {
       if (wide) sweep_spmv<TV, 2>(a.op, rw, vj, w);
       else sweep_spmv<TV, 1>(a.op, rw, vj, w);
-      block_dots<TV>(bs, w, rw, j + 1, true, sink(A, nred), S.dpart, pair);
+      block_dots<TV, RES>(bs, w, rw, j + 1, true, sink(A, nred), S.dpart, pair);
       count<TV>(S, 4.0, j + 2.0);  // w = A v_j (v_j, hx, hy, w); v_i . w (j + 1 vectors, w)
     }
     acc_settle(A, a.bar, nred, j + 3, nset);
@@ -1081,7 +1133,7 @@ __device__ SolveState krylov(const GmresArgs& a, const double* __restrict__ bvec
       if (!fused2) {
         if (wide) sweep_combine<TV, true, 2>(rw, bs, S.coef, j + 1, w, w);
         else sweep_combine<TV, true, 1>(rw, bs, S.coef, j + 1, w, w);
-        block_dots<TV>(bs, w, rw, j + 1, true, sink(A, nred), S.dpart, pair);
+        block_dots<TV, RES>(bs, w, rw, j + 1, true, sink(A, nred), S.dpart, pair);
         count<TV>(S, 3.0, 2.0 * (j + 1));  // w -= V d (j + 1 vectors, w twice); v_i . w again
       }
       acc_settle(A, a.bar, nred, j + 3, nset);
@@ -1187,7 +1239,7 @@ __device__ SolveState krylov(const GmresArgs& a, const double* __restrict__ bvec
     st.it = j + 1;
     count<TV>(S, 3.0, j + 2.0);  // v_{j+1} = (w - V coef) / nn: j + 1 vectors, w, v_{j+1}; rres read and written
     rmx = block_max(rmx, S.scratch);
-    if (threadIdx.x == 0) acc_max(A.row(nred), j + 4, rmx);  // entry (j+1)+3, read after the next sweep A
+    if (threadIdx.x == 0) acc_max(A, nred, j + 4, rmx);  // entry (j+1)+3, read after the next sweep A
   }
   // ---- x = x0 + V_k y_k for the returned iterate k ----
   if (!grid_sync(a.bar, gen, a.spin_limit)) {
@@ -1232,7 +1284,7 @@ __global__ void __launch_bounds__(NT) gmres_kernel(GmresArgs a)
   }
   if constexpr (!MIXED) {
     const SolveState st =
-        krylov<double, RES>(a, a.b, a.x0, a.x, a.V, a.w, a.r, limit > 0 ? limit : 0, a.tol, 0.0, 1, gen, nred, nset, sh);
+        krylov<double, RES>(a, a.b, a.x0, a.x, a.V, a.r, limit > 0 ? limit : 0, a.tol, 0.0, 1, gen, nred, nset, sh);
     out.iterations = st.best_it;
     out.converged = st.converged;
     out.breakdown = st.breakdown;
@@ -1260,7 +1312,7 @@ __global__ void __launch_bounds__(NT) gmres_kernel(GmresArgs a)
       const int left = limit - total;
       const bool last = cycles + 1 >= a.max_refine;
       const int kin = per_cycle < left ? per_cycle : left;
-      st = krylov<float, RES>(a, a.b, xin, a.x, a.V32, a.w, a.r, kin > 0 ? kin : 0, a.tol, last ? 0.0 : a.inner_rtol,
+      st = krylov<float, RES>(a, a.b, xin, a.x, a.V32, a.r, kin > 0 ? kin : 0, a.tol, last ? 0.0 : a.inner_rtol,
                               reorth, gen, nred, nset, sh);
       if (cycles == 0) {
         out.initial_linf = st.r0_linf;
@@ -1309,7 +1361,7 @@ __global__ void __launch_bounds__(NT) gmres_kernel(GmresArgs a)
   } else if (!out.timeout && grid_sync(a.bar, gen, a.spin_limit)) {
     const Rows rw = own_rows(a.n);
     const Smem S = carve(sh, a.m);
-    const Acc A{a.acc, a.ld, nullptr};  // maxima only
+    const Acc A{a.acc, a.ld, acc_stride(a.prow), nullptr};  // maxima only
     double rmax = 0.0, bmax = 0.0;
     for (int q = rw.r0 + threadIdx.x; q < rw.r1; q += NT) {
       const int qq[1] = {q};
@@ -1321,8 +1373,8 @@ __global__ void __launch_bounds__(NT) gmres_kernel(GmresArgs a)
     rmax = block_max(rmax, S.scratch);
     bmax = block_max(bmax, S.scratch);
     if (threadIdx.x == 0) {
-      acc_max(A.row(nred), 0, rmax);
-      acc_max(A.row(nred), 1, bmax);
+      acc_max(A, nred, 0, rmax);
+      acc_max(A, nred, 1, bmax);
     }
     if (grid_sync(a.bar, gen, a.spin_limit)) {
       if (blockIdx.x == 0) {
@@ -1428,7 +1480,7 @@ struct EcgGmresWork {
   double* r = nullptr;
   float* V32 = nullptr;
   double* part = nullptr;  // residual_kernel's block maxima
-  double* acc = nullptr;   // three accumulator rows of ld doubles
+  double* acc = nullptr;   // three accumulator rows of ld entries
   double* dpt = nullptr;   // deterministic mode: three per-block partial tables (nblocks x ld)
   int ld = 0;
   double* R = nullptr;
@@ -1439,6 +1491,7 @@ struct EcgGmresWork {
   size_t smem = 0;
   int kres = 0;  // basis vectors resident in shared memory
   int prow = 0;  // rows of a block
+  int wrows = 0; // rows of w in shared memory
 };
 
 EcgGmresWork* gmres_work_create(long long n, int max_iter, int num_sms, int device, bool mixed, std::string* err)
@@ -1482,6 +1535,14 @@ EcgGmresWork* gmres_work_create(long long n, int max_iter, int num_sms, int devi
   if (kres < 32 && kres < w->m + 1) kres = 0;
   w->kres = static_cast<int>(kres);
   w->smem = fixed + static_cast<size_t>(kres) * vbytes;
+  // Without resident vectors, large blocks keep w there where that leaves the L1
+  // cache about half of the SM's (an iteration on the bubble at 2560x640 139.6 ->
+  // 131.3 us, 768x768 FP64 136 -> 131, 512x512 64.2 -> 62.3).
+  const size_t wbytes = sizeof(double) * w->prow;
+  if (kres == 0 && w->prow > kSmallRows && wbytes <= 96u * 1024u && w->smem + wbytes <= budget) {
+    w->wrows = w->prow;
+    w->smem += wbytes;
+  }
   bool ok = true;
   auto alloc = [&](void** p, size_t bytes) {
     if (ok && cudaMalloc(p, bytes) != cudaSuccess) ok = false;
@@ -1492,7 +1553,7 @@ EcgGmresWork* gmres_work_create(long long n, int max_iter, int num_sms, int devi
   alloc(reinterpret_cast<void**>(&w->w), sizeof(double) * n);
   alloc(reinterpret_cast<void**>(&w->r), sizeof(double) * n);
   alloc(reinterpret_cast<void**>(&w->part), sizeof(double) * 2 * kResidualBlocks);
-  alloc(reinterpret_cast<void**>(&w->acc), sizeof(double) * 3 * w->ld);
+  alloc(reinterpret_cast<void**>(&w->acc), sizeof(double) * 3 * w->ld * acc_stride(w->prow));
   alloc(reinterpret_cast<void**>(&w->dpt), sizeof(double) * 3 * static_cast<size_t>(w->nblocks) * w->ld);
   alloc(reinterpret_cast<void**>(&w->R), sizeof(double) * (w->m + 1) * (w->m + 1));
   alloc(reinterpret_cast<void**>(&w->bar), sizeof(GridBar));
@@ -1577,10 +1638,11 @@ cudaError_t gmres_enqueue(EcgGmresWork* w, const EcgPressureOp& op, const double
   a.reorth = reorth;
   a.kres = w->kres;
   a.prow = w->prow;
+  a.wrows = w->wrows;
   a.spin_limit = 1LL << 25;  // ~2 s of polling before a barrier gives up
   cudaError_t e = cudaMemsetAsync(w->bar, 0, sizeof(GridBar), s);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(w->acc, 0, sizeof(double) * 3 * w->ld, s);
+  e = cudaMemsetAsync(w->acc, 0, sizeof(double) * 3 * w->ld * acc_stride(w->prow), s);
   if (e != cudaSuccess) return e;
   void* args[] = {&a};
   return cudaLaunchCooperativeKernel(gmres_entry(w->kres > 0, w->mixed), dim3(w->nblocks), dim3(NT), args, w->smem, s);
