@@ -1,21 +1,28 @@
-// Default explicit step of the fast build: warps march up column strips.
-// Included inside the ecg_fast namespace of stencil.cuh, after fv_fast.cuh
-// (it uses that file's Newton-refined arithmetic and flux functions).
+// Default explicit step: warps march up column strips.  Included inside the
+// arithmetic namespace of stencil.cuh, after fv_fast.cuh (the fast build's
+// Newton-refined arithmetic and flux functions) or fv_exact.cuh (the exact
+// build's, under the same names).
 //
 // A warp owns the 28 cells [c0, c0+28) of a row strip; lane l holds column
 // c0 - 2 + l (lanes 0-1 and 30-31 carry the MUSCL halo).  It walks rows
-// j0 .. j0+H-1 keeping, per lane, the primitives of rows j-1 .. j+2 in
-// registers:
-//   * x-neighbours for the x-slopes and x-face states come by warp shuffles;
+// j0 .. j0+H-1:
 //   * the y-slope of a row is computed once and reused by both y-faces;
 //   * the y-face flux above row j becomes the flux below row j+1 without
 //     leaving registers.
 // Every face flux is evaluated once per warp strip (the x-face at a strip
-// edge by both strips), with no shared memory and no block barrier in the
-// loop.  Reductions (CFL rate, admissibility, degenerate count) accumulate in
-// registers and are committed once per block.
+// edge by both strips), with no block barrier in the loop.  Reductions (CFL
+// rate, admissibility, degenerate count) accumulate in registers and are
+// committed once per block.
+// Two forms: rows through shared memory (march_strip_staged, the default), and
+// rows j-1 .. j+2 in registers with the x-neighbours by warp shuffles
+// (march_strip, the fast build's tile_y 2 and 3).
 namespace march {
 
+#ifdef ECG_FAST_KERNEL
+constexpr bool kExact = false;
+#else
+constexpr bool kExact = true;
+#endif
 constexpr int kLanes = 32;
 constexpr int kCells = 28;  // interior cells per warp strip
 
@@ -34,6 +41,7 @@ __device__ __forceinline__ Prim slope3(const Prim& m, const Prim& c, const Prim&
               fast::slope_f(c.v - m.v, p.v - c.v, LIM), fast::slope_f(c.p - m.p, p.p - c.p, LIM)};
 }
 
+// (0.5 s is exact, so the fused form rounds like q + 0.5 s in either build)
 __device__ __forceinline__ Prim plus_half(const Prim& q, const Prim& s)
 {
   return Prim{fma(0.5, s.rho, q.rho), fma(0.5, s.u, q.u), fma(0.5, s.v, q.v), fma(0.5, s.p, q.p)};
@@ -483,10 +491,18 @@ __device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const d
     const Cons fr{shdn(fl.rho), shdn(fl.mx), shdn(fl.my), shdn(fl.E)};
     const Cons old = conserved(j);
     Cons n;
-    n.rho = old.rho - fma(dtx, fr.rho - fl.rho, dty * (gt.rho - gb.rho));
-    n.mx = old.mx - fma(dtx, fr.mx - fl.mx, dty * (gt.mx - gb.mx));
-    n.my = old.my - fma(dtx, fr.my - fl.my, dty * (gt.my - gb.my));
-    n.E = old.E - fma(dtx, fr.E - fl.E, dty * (gt.E - gb.E));
+    if constexpr (kExact) {
+      const double idx = P.g.inv_dx, idy = P.g.inv_dy;
+      n.rho = old.rho - dt * ((fr.rho - fl.rho) * idx + (gt.rho - gb.rho) * idy);
+      n.mx = old.mx - dt * ((fr.mx - fl.mx) * idx + (gt.mx - gb.mx) * idy);
+      n.my = old.my - dt * ((fr.my - fl.my) * idx + (gt.my - gb.my) * idy);
+      n.E = old.E - dt * ((fr.E - fl.E) * idx + (gt.E - gb.E) * idy);
+    } else {
+      n.rho = old.rho - fma(dtx, fr.rho - fl.rho, dty * (gt.rho - gb.rho));
+      n.mx = old.mx - fma(dtx, fr.mx - fl.mx, dty * (gt.mx - gb.mx));
+      n.my = old.my - fma(dtx, fr.my - fl.my, dty * (gt.my - gb.my));
+      n.E = old.E - fma(dtx, fr.E - fl.E, dty * (gt.E - gb.E));
+    }
     gb = gt;
     const Prim q = fast::to_prim_f(n, g);
     const double cs = fast::fsound_w(q.rho, q.p, g);
@@ -497,7 +513,8 @@ __device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const d
       o[3 * pl] = n.E;
       // running extrema as doubles: the comparisons skip a NaN as the keys'
       // NaN test does, and a strip with a bad cell takes the floor at its end
-      const double rate = (fabs(q.u) + cs) * P.g.inv_dx + (fabs(q.v) + cs) * P.g.inv_dy;
+      const double rate = kExact ? (fabs(q.u) + cs) / P.g.dx + (fabs(q.v) + cs) / P.g.dy
+                                 : (fabs(q.u) + cs) * P.g.inv_dx + (fabs(q.v) + cs) * P.g.inv_dy;
       rate_max = rate > rate_max ? rate : rate_max;
       rho_min = q.rho < rho_min ? q.rho : rho_min;
       p_min = q.p < p_min ? q.p : p_min;
@@ -519,9 +536,10 @@ __device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const d
 // registers, without a spill, beat 12 for the HLLC fluxes on large grids
 // (2048x2048 132 against 137 us, 2560x640 equal), 20 at 96 registers spill and
 // lose (164 us, 70 us); the XIE flux (2560x640: 104 us at 12, 116 at 16) and
-// Rusanov, which spills at 128, stay at 12.
+// Rusanov, which spills at 128, stay at 12, as does the exact build, whose IEEE
+// divisions and square roots spill at 128 (1280x320 33.4 us at 16, 31.9 at 12).
 template <int RK>
-constexpr int kStagedWarps = RK == ECG_RIEMANN_HLLC || RK == ECG_RIEMANN_LOWMACH_HLLC ? 16 : 12;
+constexpr int kStagedWarps = !kExact && (RK == ECG_RIEMANN_HLLC || RK == ECG_RIEMANN_LOWMACH_HLLC) ? 16 : 12;
 
 // The register-loaded strips take at most 128 registers a thread (16 warps
 // per SM), measured faster than the 166-register schedule the paired faces get
@@ -622,6 +640,20 @@ cudaError_t launch_rk(const EcgFvParams& p, const double* in, double* out, EcgSt
   }
 }
 
+#ifndef ECG_FAST_KERNEL
+// Exact build, every flux but XIE (launch_fv_step): 1280x320 HLLC 31.9 us
+// against 42.8 on the 32x16 tiles, 2560x640 105 against 165, 128x128 7.1
+// against 14.7.
+inline cudaError_t launch(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats,
+                          const EcgDtCtl& ctl, cudaStream_t s)
+{
+  switch (p.riemann) {
+    case ECG_RIEMANN_RUSANOV: return launch_rk<ECG_RIEMANN_RUSANOV, true, true>(p, in, out, stats, ctl, s);
+    case ECG_RIEMANN_LOWMACH_HLLC: return launch_rk<ECG_RIEMANN_LOWMACH_HLLC, true, true>(p, in, out, stats, ctl, s);
+    default: return launch_rk<ECG_RIEMANN_HLLC, true, true>(p, in, out, stats, ctl, s);
+  }
+}
+#else
 template <int RK>
 cudaError_t launch_mode(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats, const EcgDtCtl& ctl,
                         cudaStream_t s, bool pair, bool stage)
@@ -657,5 +689,7 @@ inline cudaError_t launch(const EcgFvParams& p, const double* in, double* out, E
     default: return launch_mode<ECG_RIEMANN_HLLC>(p, in, out, stats, ctl, s, pair, stage);
   }
 }
+
+#endif
 
 }  // namespace march

@@ -472,7 +472,7 @@ cudaError_t launch_fv_rk(const EcgFvParams& p, const double* in, double* out, Ec
                          const EcgDtCtl& ctl, int tile_y, cudaStream_t s)
 {
   if (tile_y == 8) return launch_fv_t<RK, 8>(p, in, out, stats, ctl, s);
-  // 0 (default) in the exact build, 16: the 32x16 tile
+  // 16, and the exact build's XIE flux: the 32x16 tile
   return launch_fv_t<RK, 16>(p, in, out, stats, ctl, s);
 }
 
@@ -480,6 +480,9 @@ cudaError_t launch_fv_rk(const EcgFvParams& p, const double* in, double* out, Ec
 #include "fv_fast.cuh"
 #include "fv_march.cuh"
 #include "fv_batch.cuh"
+#else
+#include "fv_exact.cuh"
+#include "fv_march.cuh"
 #endif
 
 cudaError_t launch_fv_step(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats,
@@ -494,6 +497,11 @@ cudaError_t launch_fv_step(const EcgFvParams& p, const double* in, double* out, 
   if (tile_y == 3) return march::launch(p, in, out, stats, ctl, s, true, false);
   if (tile_y == 2) return march::launch(p, in, out, stats, ctl, s, false, false);
   if (tile_y == 1) return fast::launch(p, in, out, stats, ctl, s);
+#else
+  // 8 or 16: a 32xTY tile; else column strips, but for the XIE flux, whose
+  // out-of-line evaluation costs the strips more than the tiles (1280x320: 99
+  // against 89 us)
+  if (tile_y != 8 && tile_y != 16 && p.riemann != ECG_RIEMANN_XIE_AM_HLLC_P) return march::launch(p, in, out, stats, ctl, s);
 #endif
   switch (p.riemann) {
     case ECG_RIEMANN_RUSANOV: return launch_fv_rk<ECG_RIEMANN_RUSANOV>(p, in, out, stats, ctl, tile_y, s);
