@@ -924,20 +924,23 @@ static ecg_status run_explicit(ecg_ctx* c, int32_t max_step, double stop_time, e
     ctl.reset_slot = -1;
     ctl.cfl = c->cfg.cfl;
     ctl.stop_time = stop_time;
-    // capture (or reuse) the chunk graph for this buffer parity and step base
+    // capture (or reuse) the chunk graph for this buffer parity and step base;
+    // no launches past the step limit (a stopped step is a launch all the same)
+    const int nodes = std::max(1, std::min(K, max_step - steps));
     ecg_ctx::Graph* gr = nullptr;
     for (auto& g : c->graphs) {
-      if (g.cur == c->cur && g.max_step == max_step && g.stop_time == stop_time) gr = &g;
+      if (g.cur == c->cur && g.nodes == nodes && g.max_step == max_step && g.stop_time == stop_time) gr = &g;
     }
     if (!gr) {
       c->graphs.push_back(ecg_ctx::Graph());
       gr = &c->graphs.back();
       gr->cur = c->cur;
+      gr->nodes = nodes;
       gr->max_step = max_step;
       gr->stop_time = stop_time;
       cudaGraph_t graph;
       if (!cuda_ok(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "capture")) return ECG_ERR_CUDA;
-      for (int k = 0; k < K; ++k) {
+      for (int k = 0; k < nodes; ++k) {
         const double* in = c->d_state[(c->cur + k) & 1];
         double* o = c->d_state[(c->cur + k + 1) & 1];
         fill_ring(c, in, 0.0, c->d_stats, k);
@@ -953,12 +956,12 @@ static ecg_status run_explicit(ecg_ctx* c, int32_t max_step, double stop_time, e
       if (!cuda_ok(c, ie, "instantiate")) return ECG_ERR_CUDA;
     }
     if (!cuda_ok(c, cudaGraphLaunch(gr->exec, c->stream), "graph launch")) return ECG_ERR_CUDA;
-    if (!cuda_ok(c, cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(EcgStepStats) * (K + 1), cudaMemcpyDeviceToHost,
+    if (!cuda_ok(c, cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(EcgStepStats) * (nodes + 1), cudaMemcpyDeviceToHost,
                                     c->stream), "copy stats"))
       return ECG_ERR_CUDA;
     if (!cuda_ok(c, cudaStreamSynchronize(c->stream), "sync")) return ECG_ERR_CUDA;
     int ran = 0;
-    for (int k = 0; k < K; ++k) {
+    for (int k = 0; k < nodes; ++k) {
       const EcgStepStats& s = c->h_stats[k];
       if (!s.ran) break;
       ++ran;
@@ -974,13 +977,17 @@ static ecg_status run_explicit(ecg_ctx* c, int32_t max_step, double stop_time, e
     out->diagnostics.rho_min = okey_to_double(last.rho_min_key);
     out->diagnostics.pressure_min = okey_to_double(last.p_min_key);
     out->diagnostics.nonfinite_count = last.nonfinite;
-    if (ran < K) {
+    if (ran < nodes) {
       out->failure_code = last.failure;
       out->failed = last.failure != 0;
       break;
     }
+    // at a limit the loop stops here: a launch would only find the same (the
+    // checks of the final state follow below), 32 launches for nothing when the
+    // limit falls on a chunk's end
+    if (steps >= max_step || !(t < stop_time - 1.0e-14)) break;
     // the next chunk starts from the record of its first state; slots 1..K reset
-    if (!cuda_ok(c, cudaMemcpyAsync(c->d_stats, c->d_stats + K, sizeof(EcgStepStats), cudaMemcpyDeviceToDevice,
+    if (!cuda_ok(c, cudaMemcpyAsync(c->d_stats, c->d_stats + nodes, sizeof(EcgStepStats), cudaMemcpyDeviceToDevice,
                                     c->stream), "carry"))
       return ECG_ERR_CUDA;
     if (!cuda_ok(c, c->ops->init_stats(c->d_stats + 1, K, 0.0, c->stream), "init stats")) return ECG_ERR_CUDA;

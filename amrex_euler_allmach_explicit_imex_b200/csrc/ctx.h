@@ -58,6 +58,7 @@ struct ecg_ctx {
 
   struct Graph {
     int cur = 0;
+    int nodes = 0;  // steps in the graph
     int max_step = 0;
     double stop_time = 0.0;
     cudaGraphExec_t exec = nullptr;

@@ -2,8 +2,7 @@
 // advanced by one persistent launch per step.  Included inside the ecg_fast
 // namespace of stencil.cuh after fv_march.cuh (it reuses march_strip_staged:
 // the rows of each warp strip come through the warp's shared-memory ring, as
-// in the single-grid default; 20.3 against 17.4 G cell-updates/s with the
-// rows in registers on the 64-solve bench batch).
+// in the single-grid default).
 //
 // The solves' work is cut into tiles of WPB warp strips x H rows; tile
 // indices run over all solves (EcgBatchSolve::tile0 is the prefix sum).  A
@@ -59,8 +58,10 @@ __device__ __forceinline__ bool solve_control(EcgStepStats* __restrict__ st, con
   return !halt;
 }
 
+// 12 warps per SM and no spill: the 64-solve batch 208 us a step against 222 with
+// the single-grid strips' 16, at which this kernel's solve record spills.
 template <int RK, int LIM, int H, int WPB>
-__global__ void __launch_bounds__(WPB * 32, march::kStagedWarps<RK> / WPB)
+__global__ void __launch_bounds__(WPB * 32, 12 / WPB)
 fv_batch_kernel(const EcgBatchSolve* __restrict__ solves, EcgStepStats* __restrict__ stats,
                 unsigned long long* __restrict__ degenerate_total, const int* __restrict__ max_step,
                 const EcgBatchCtl ctl)
@@ -95,8 +96,13 @@ fv_batch_kernel(const EcgBatchSolve* __restrict__ solves, EcgStepStats* __restri
     march::MarchAcc acc;
     acc.init();
     if (c0 < S.p.g.nx)
-      march::march_strip_staged<RK, LIM>(S.p, S.u[par], S.u[par ^ 1], c0, j0, H, s_dt,
-                                               ctl.count_degenerate != 0, acc, ring[warp]);
+      march::march_strip_staged<RK, LIM>(
+          S.p, S.u[par], S.u[par ^ 1], c0, j0, H,
+          [&](double& dt) {
+            dt = s_dt;
+            return true;
+          },
+          ctl.count_degenerate != 0, acc, ring[warp]);
     const int deg = block_commit<WPB * 32>(red, acc.kmax, acc.krho, acc.kp, acc.nonfinite, acc.degenerate,
                                            &stats[3 * s + ctl.acc_slot]);
     if (threadIdx.x == 0 && deg != 0) atomicAdd(&degenerate_total[s], static_cast<unsigned long long>(deg));

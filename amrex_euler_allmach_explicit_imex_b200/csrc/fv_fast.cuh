@@ -468,8 +468,7 @@ fv_fast_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
   const int nx = P.g.nx, ny = P.g.ny;
   const double g = P.gamma, inv_gm1 = frcp(g - 1.0);
 
-  double dt;
-  if (!step_control(stats, ctl, dt)) return;
+  loop_wait();
 
   auto R = [](int x, int y) { return (y + 2) * RW + (x + 2); };
   auto SI = [](int x, int y) { return (y + 1) * SW + (x + 1); };
@@ -482,7 +481,11 @@ fv_fast_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
     q_v[e] = q.v;
     q_p[e] = q.p;
   }
+  // (the control's chain of loads and divisions runs beside the tile's loads)
+  double dt;
+  const bool go = step_control(stats, ctl, dt);
   __syncthreads();
+  if (!go) return;
 
   // ---- limited slopes, both axes, cells [-1, T]^2 ----
   const int lim = P.limiter;
@@ -643,6 +646,7 @@ fv_fast_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
       if (ctl.count_degenerate && deg) degenerate += wb + wt;
     }
   }
+  loop_ready();
   __syncthreads();  // every slope / primitive read is done: reuse the slope region
   double* F = sl;             // 4 planes of NF x-face fluxes
   double* G = sl + 4 * NF;    // 4 planes of NF y-face fluxes
@@ -705,8 +709,7 @@ cudaError_t launch_rk(const EcgFvParams& p, const double* in, double* out, EcgSt
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
   const dim3 grid((p.g.nx + T - 1) / T, (p.g.ny + T - 1) / T);
-  kern<<<grid, S::NT, S::bytes, s>>>(p, in, out, stats, ctl);
-  return cudaGetLastError();
+  return launch_loop(ctl.device_dt != 0, kern, grid, S::NT, S::bytes, s, p, in, out, stats, ctl);
 }
 
 inline cudaError_t launch(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats,

@@ -287,9 +287,12 @@ __device__ __forceinline__ Cons face_xie(const Prim& l, const Prim& r, int axis,
 // it needs come along the march: the y-faces' below and above row j (carried,
 // and this row's), and the x-faces' of rows j and j+1 (row j+1's from the
 // pressure of the window's next row, carried on).
-template <int RK, int LIM>
-__device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const double* __restrict__ u,
-                                                   double* __restrict__ out, int c0, int j0, int H, double dt,
+// control(dt) gives the step's dt, or false to stop, after the first rows have
+// been requested: its chain of loads and divisions runs beside theirs.  Returns
+// what it returned.
+template <int RK, int LIM, class Control>
+__device__ __forceinline__ bool march_strip_staged(const EcgFvParams& P, const double* __restrict__ u,
+                                                   double* __restrict__ out, int c0, int j0, int H, Control control,
                                                    bool count_deg, MarchAcc& acc, StageRing& ring)
 {
   constexpr bool XIE = RK == ECG_RIEMANN_XIE_AM_HLLC_P;
@@ -304,7 +307,6 @@ __device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const d
   const int rhi = P.row_hi > 0 && P.row_hi < ny ? P.row_hi : ny;
   const int jend = j0 + H < rhi ? j0 + H : rhi;
   const int jlast = jend + 1;  // the last row the strip reads
-  const double dtx = dt * P.g.inv_dx, dty = dt * P.g.inv_dy;
 
   double* const col = &ring.v[0][0][lane];
   double* const qcol = &ring.q[0][0][lane];
@@ -391,6 +393,12 @@ __device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const d
   // ---- prologue: stage rows j0-2 .. j0+1+kAhead; rows j0-2 .. j0+1 first ----
 #pragma unroll
   for (int r = -2; r <= 1 + kAhead; ++r) put(j0 + r);
+  double dt;
+  if (!control(dt)) {
+    cp_async_wait<0>();
+    return false;
+  }
+  const double dtx = dt * P.g.inv_dx, dty = dt * P.g.inv_dy;
   cp_async_wait<kAhead>();
   Prim yp;  // row j's state at its upper y-face
   Cons gb;  // the y-face below row j
@@ -529,6 +537,7 @@ __device__ __forceinline__ void march_strip_staged(const EcgFvParams& P, const d
   acc.kmax = umax64(acc.kmax, okey(rate_max));
   acc.krho = umin64(acc.krho, okey(rho_min));
   acc.kp = umin64(acc.kp, okey(p_min));
+  return true;
 }
 
 // Resident warps per SM the staged strips are compiled for.  They need 146 to
@@ -557,18 +566,23 @@ fv_march_kernel(const EcgFvParams P, const double* __restrict__ u, double* __res
   const int c0 = strip * kCells;
   const int j0 = (P.row_hi > 0 ? P.row_lo : 0) + blockIdx.y * H;
 
-  double dt;
-  if (!step_control(stats, ctl, dt)) return;
+  loop_wait();
+  auto control = [&](double& dt) { return step_control(stats, ctl, dt); };
 
   MarchAcc acc;
   acc.init();
-  if (c0 < P.g.nx) {
-    if constexpr (STAGE)
-      march_strip_staged<RK, LIM>(P, u, out, c0, j0, H, dt, ctl.count_degenerate != 0, acc,
-                                        ring[STAGE ? threadIdx.x >> 5 : 0]);
-    else
-      march_strip<RK, LIM, PAIR>(P, u, out, c0, j0, H, dt, ctl.count_degenerate != 0, acc);
+  double dt;
+  if constexpr (STAGE) {
+    // (a stop is the same for every warp of the launch)
+    const bool go = c0 < P.g.nx ? march_strip_staged<RK, LIM>(P, u, out, c0, j0, H, control, ctl.count_degenerate != 0,
+                                                              acc, ring[threadIdx.x >> 5])
+                                : control(dt);
+    if (!go) return;
+  } else {
+    if (!control(dt)) return;
+    if (c0 < P.g.nx) march_strip<RK, LIM, PAIR>(P, u, out, c0, j0, H, dt, ctl.count_degenerate != 0, acc);
   }
+  loop_ready();
   block_commit<WPB * 32>(red, acc.kmax, acc.krho, acc.kp, acc.nonfinite, acc.degenerate, &stats[ctl.acc_slot]);
 }
 
@@ -625,8 +639,8 @@ cudaError_t launch_lim(const EcgFvParams& p, const double* in, double* out, EcgS
     H = rows_per_warp(rows, bx, static_cast<long long>(p.sm_count > 0 ? p.sm_count : 148) * blocks_per_sm);
   }
   const dim3 grid(bx, (rows + H - 1) / H);
-  fv_march_kernel<RK, LIM, WPB, PAIR, STAGE><<<grid, WPB * 32, 0, s>>>(p, in, out, stats, ctl, H);
-  return cudaGetLastError();
+  return launch_loop(ctl.device_dt != 0, fv_march_kernel<RK, LIM, WPB, PAIR, STAGE>, grid, WPB * 32, 0, s, p, in, out,
+                     stats, ctl, H);
 }
 
 template <int RK, bool PAIR, bool STAGE>
@@ -672,17 +686,16 @@ inline cudaError_t launch(const EcgFvParams& p, const double* in, double* out, E
     case ECG_RIEMANN_RUSANOV: return launch_mode<ECG_RIEMANN_RUSANOV>(p, in, out, stats, ctl, s, pair, stage);
     case ECG_RIEMANN_LOWMACH_HLLC: return launch_mode<ECG_RIEMANN_LOWMACH_HLLC>(p, in, out, stats, ctl, s, pair, stage);
     case ECG_RIEMANN_XIE_AM_HLLC_P: {
-      // Staged strips carry the 5-face sensor along, on grids whose strips
-      // fill a wave of resident warps with runs of 8 rows or more (2560x640:
-      // 139 us against the tile kernel's 176 us), and for a band of rows
-      // (the pipelined host step: the tile kernel steps whole grids only);
-      // smaller grids, and the other variants, use the 16x16 tile kernel
-      // (Gresho 256^2: 19 us against 34 us on strips).
-      const long long strips = (p.g.nx + kCells - 1) / kCells;
-      const int rlo = p.row_hi > 0 ? p.row_lo : 0;
-      const int rhi = p.row_hi > 0 && p.row_hi < p.g.ny ? p.row_hi : p.g.ny;
-      const long long slots = static_cast<long long>(p.sm_count > 0 ? p.sm_count : 148) * 12;
-      if (stage && (p.row_hi > 0 || strips * ((rhi - rlo + 7) / 8) >= slots))
+      // Staged strips carry the 5-face sensor along (2560x640 104 us against
+      // the tile kernel's 150, 512x512 22.5 against 28.0, 128x128 7.2 against
+      // 8.9); on grids of one to three 16x16 tiles an SM, where the strips
+      // are too few and short and the tiles run as one wave, the tile kernel is
+      // the faster (256x256 10.4 against 11.2, 333x331 12.8 against 14.0;
+      // 512x256, 512 tiles, 18.1 against 14.2).  A band of rows (the pipelined
+      // host step) takes the strips: the tile kernel steps whole grids only.
+      const long long tiles = static_cast<long long>((p.g.nx + 15) / 16) * ((p.g.ny + 15) / 16);
+      const long long sms = p.sm_count > 0 ? p.sm_count : 148;
+      if (stage && (p.row_hi > 0 || tiles <= sms || tiles > 3 * sms))
         return launch_rk<ECG_RIEMANN_XIE_AM_HLLC_P, false, true>(p, in, out, stats, ctl, s);
       return fast::launch(p, in, out, stats, ctl, s);
     }

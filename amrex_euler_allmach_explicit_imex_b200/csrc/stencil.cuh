@@ -20,6 +20,37 @@ constexpr double kInf = __builtin_huge_val();
 constexpr double kLowest = -1.7976931348623157e308;
 constexpr double kMax = 1.7976931348623157e308;
 
+// ---- launches of the device loop ------------------------------------------------
+// The steps of a device loop follow one another in a graph, each reading what the
+// one before wrote.  Launched with programmatic serialisation, a kernel's blocks
+// are scheduled once every block of its predecessor has come to loop_ready (at
+// the end of its faces: earlier, the successor's blocks take slots on the SMs
+// that have the fewest and the load tilts, 256x256 14.8 against 13.9 us a step)
+// and wait at loop_wait for its completion and its writes, so the launch leaves
+// the chain: HLLC 256x256 11.5 -> 10.0 us a step, 400x4 with its ring 11.2 -> 9.6,
+// 2560x640 65.5 -> 63.2 (host waits and set-up of a 32-step run included; the
+// last with the empty launches after the step limit gone too).  Nothing of the
+// state or the records is read before loop_wait.
+__device__ __forceinline__ void loop_ready() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void loop_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_loop(bool loop, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s,
+                        A... args)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = loop ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // ---- boundary-aware cell loads ---------------------------------------------
 
 __device__ __forceinline__ int wrapi(int i, int n)
@@ -310,6 +341,7 @@ fv_step_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
   const int nx = P.g.nx, ny = P.g.ny;
 
   double dt;
+  loop_wait();
   if (!step_control(stats, ctl, dt)) return;
 
   // ---- phase A: halo region -> primitives in shared memory ----
@@ -405,6 +437,7 @@ fv_step_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
   }
   __syncthreads();
 
+  loop_ready();
   // ---- phase C: conservative update + fused reductions ----
   unsigned long long kmax = okey(kLowest), krho = okey(kMax), kp = okey(kMax);
   int nonfinite = 0;
@@ -463,8 +496,7 @@ cudaError_t launch_fv_t(const EcgFvParams& p, const double* in, double* out, Ecg
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(S::bytes));
   if (e != cudaSuccess) return e;
   const dim3 grid((p.g.nx + TX - 1) / TX, (p.g.ny + TY - 1) / TY);
-  kern<<<grid, NT, S::bytes, s>>>(p, in, out, stats, ctl);
-  return cudaGetLastError();
+  return launch_loop(ctl.device_dt != 0, kern, grid, NT, S::bytes, s, p, in, out, stats, ctl);
 }
 
 template <int RK>
@@ -805,6 +837,8 @@ __global__ void ghost_box_kernel(const EcgFvParams P, const EcgProblem pr, const
                                  const EcgStepStats* __restrict__ stats, int k, double* __restrict__ out,
                                  long long opitch, long long oplane, int only_ring)
 {
+  loop_ready();
+  loop_wait();
   if (stats != nullptr) time = stats[k].t;
   const int nx = P.g.nx, ny = P.g.ny, W = nx + 4, H = ny + 4;
   const int n = only_ring ? 4 * W + 4 * ny : W * H;
@@ -865,8 +899,8 @@ cudaError_t launch_ghost_box(const EcgFvParams& p, const EcgProblem& pr, const d
 {
   const long long w = p.g.nx + 4;
   const long long n = only_ring ? 4 * (w + p.g.ny) : w * (p.g.ny + 4);
-  ghost_box_kernel<<<reduce_blocks(n, 256), 256, 0, s>>>(p, pr, u, time, stats, k, out, opitch, oplane, only_ring);
-  return cudaGetLastError();
+  return launch_loop(stats != nullptr, ghost_box_kernel, dim3(reduce_blocks(n, 256)), 256, 0, s, p, pr, u, time, stats,
+                     k, out, opitch, oplane, only_ring);
 }
 
 cudaError_t launch_riemann_star(const EcgProblem& pr, double* out, cudaStream_t s)
