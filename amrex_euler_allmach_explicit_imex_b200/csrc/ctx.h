@@ -106,6 +106,7 @@ bool fetch_fused(ecg_ctx* c);
 // the context's pinned staging buffers
 bool host_pageable(const void* p);
 HostStage* host_stage(ecg_ctx* c);  // null when the pinned buffers cannot be allocated (c->err set)
+HostStage* host_stage_sized(HostStage* s, size_t doubles, bool to_device);  // s or a new one, its buffer for the direction made
 void host_stage_destroy(HostStage* s);
 double* host_stage_in(HostStage* s);
 double* host_stage_out(HostStage* s);

@@ -128,6 +128,33 @@ bool host_pageable(const void* p)
   return a.type == cudaMemoryTypeUnregistered;
 }
 
+// three quarters of the host threads, with the caller (measured on a 16-thread
+// host at 2560x640: 3, 7, 11, 15 workers gave 0.40, 0.51, 0.62, 0.57 G
+// cell-updates/s through the host step)
+static CopyPool* new_pool()
+{
+  const unsigned hw = std::thread::hardware_concurrency();
+  return new CopyPool(std::max(1, std::min(15, static_cast<int>(hw * 3 / 4) - 1)));
+}
+
+// A stage of its own with room for `doubles`, for one direction at a time
+// (host_stage_in: to the device, else host_stage_out); null when the pinned
+// buffer cannot be allocated.
+HostStage* host_stage_sized(HostStage* s, size_t doubles, bool to_device)
+{
+  if (!s) {
+    s = new HostStage();
+    s->doubles = doubles;
+    s->pool = new_pool();
+  }
+  double*& buf = to_device ? s->in : s->out;
+  if (!buf && cudaMallocHost(&buf, sizeof(double) * s->doubles) != cudaSuccess) {
+    cudaGetLastError();
+    buf = nullptr;
+  }
+  return s;
+}
+
 HostStage* host_stage(ecg_ctx* c)
 {
   const size_t need = 4 * static_cast<size_t>(c->grid.nx) * static_cast<size_t>(c->grid.ny);
@@ -143,12 +170,7 @@ HostStage* host_stage(ecg_ctx* c)
     delete s;
     return nullptr;
   }
-  // three quarters of the host threads, with the caller (measured on a 16-thread
-  // host at 2560x640: 3, 7, 11, 15 workers gave 0.40, 0.51, 0.62, 0.57 G
-  // cell-updates/s through the host step)
-  const unsigned hw = std::thread::hardware_concurrency();
-  const int workers = std::max(1, std::min(15, static_cast<int>(hw * 3 / 4) - 1));
-  s->pool = new CopyPool(workers);
+  s->pool = new_pool();
   c->stage = s;
   return s;
 }

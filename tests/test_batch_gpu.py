@@ -103,3 +103,17 @@ def test_batch_rejects_mixed_solvers(gpu):
     cfgs[1] = read_config("amr.n_cell=32 8\neuler.problem=toro1\neuler.riemann=rusanov\n")
     with pytest.raises(EcgError):
         api.Batch(cfgs)
+
+
+@pytest.mark.parametrize("grid", [(255, 128), (256, 128), (2048, 16), (8193, 4), (601, 3000)])
+def test_large_pageable_boxes_cross_unchanged(gpu, grid):
+    """Solves either side of the staged-transfer size, and rows that do not
+    divide into bands, come back bit for bit (no step taken)."""
+    cfgs, states = workloads.riemann_batch(2, seed=3, grids=[grid])
+    states = [s + 1.0e-3 * np.random.default_rng(k).standard_normal(s.shape) for k, s in enumerate(states)]
+    with api.Batch(cfgs) as b:
+        for _ in range(2):
+            for k, u in enumerate(states):
+                b.upload(k, u)
+            for k, u in enumerate(states):
+                assert np.array_equal(b.download(k), u)
