@@ -674,11 +674,11 @@ fv_fast_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
       const int xl = y * (T + 1) + x, yb = y * T + x;
       const double idx = P.g.inv_dx, idy = P.g.inv_dy;
       Cons n;
-      n.rho = __ldg(u + o) - dt * ((F[xl + 1] - F[xl]) * idx + (G[yb + T] - G[yb]) * idy);
-      n.mx = __ldg(u + o + pl) - dt * ((F[NF + xl + 1] - F[NF + xl]) * idx + (G[NF + yb + T] - G[NF + yb]) * idy);
-      n.my = __ldg(u + o + 2 * pl) -
+      n.rho = load_coherent(u + o) - dt * ((F[xl + 1] - F[xl]) * idx + (G[yb + T] - G[yb]) * idy);
+      n.mx = load_coherent(u + o + pl) - dt * ((F[NF + xl + 1] - F[NF + xl]) * idx + (G[NF + yb + T] - G[NF + yb]) * idy);
+      n.my = load_coherent(u + o + 2 * pl) -
              dt * ((F[2 * NF + xl + 1] - F[2 * NF + xl]) * idx + (G[2 * NF + yb + T] - G[2 * NF + yb]) * idy);
-      n.E = __ldg(u + o + 3 * pl) -
+      n.E = load_coherent(u + o + 3 * pl) -
             dt * ((F[3 * NF + xl + 1] - F[3 * NF + xl]) * idx + (G[3 * NF + yb + T] - G[3 * NF + yb]) * idy);
       out[o] = n.rho;
       out[o + pl] = n.mx;

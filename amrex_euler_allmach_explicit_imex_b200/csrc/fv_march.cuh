@@ -192,10 +192,10 @@ __device__ __forceinline__ void march_strip(const EcgFvParams& P, const double* 
     const long long o = static_cast<long long>(j) * P.g.pitch + xs;
     const long long pl = P.g.plane;
     Cons n;
-    n.rho = __ldg(u + o) - dt * ((fr.rho - fl.rho) * idx + (gt.rho - gb.rho) * idy);
-    n.mx = __ldg(u + o + pl) - dt * ((fr.mx - fl.mx) * idx + (gt.mx - gb.mx) * idy);
-    n.my = __ldg(u + o + 2 * pl) - dt * ((fr.my - fl.my) * idx + (gt.my - gb.my) * idy);
-    n.E = __ldg(u + o + 3 * pl) - dt * ((fr.E - fl.E) * idx + (gt.E - gb.E) * idy);
+    n.rho = load_coherent(u + o) - dt * ((fr.rho - fl.rho) * idx + (gt.rho - gb.rho) * idy);
+    n.mx = load_coherent(u + o + pl) - dt * ((fr.mx - fl.mx) * idx + (gt.mx - gb.mx) * idy);
+    n.my = load_coherent(u + o + 2 * pl) - dt * ((fr.my - fl.my) * idx + (gt.my - gb.my) * idy);
+    n.E = load_coherent(u + o + 3 * pl) - dt * ((fr.E - fl.E) * idx + (gt.E - gb.E) * idy);
     const Prim q = fast::to_prim_f(n, g);
     const double cs = fast::fsound_w(q.rho, q.p, g);
     if (cell_ok) {

@@ -31,8 +31,22 @@ constexpr double kMax = 1.7976931348623157e308;
 // 2560x640 65.5 -> 63.2 (host waits and set-up of a 32-step run included; the
 // last with the empty launches after the step limit gone too).  Nothing of the
 // state or the records is read before loop_wait.
+//
+// A kernel launched this way is resident while its predecessor still writes the
+// state, the ghost ring and the records, so none of them is read-only for its
+// lifetime: they are read with coherent loads (load_coherent, cp.async, plain
+// loads of the records), never through __ldg, whose path asks for data that no
+// one writes while the kernel runs and may keep a line from before the wait.
 __device__ __forceinline__ void loop_ready() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void loop_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// (volatile: not moved across loop_wait, which is volatile too)
+__device__ __forceinline__ double load_coherent(const double* p)
+{
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
 
 template <class... P, class... A>
 cudaError_t launch_loop(bool loop, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s,
@@ -133,7 +147,7 @@ __device__ __forceinline__ Cons load_cell(const EcgFvParams& P, const double* __
 {
   const CellSrc c = cell_src(P, u, i, j);
   if (!c.p) return Cons{P.bc.cst[0], P.bc.cst[1], P.bc.cst[2], P.bc.cst[3]};
-  Cons r{__ldg(c.p), __ldg(c.p + c.pl), __ldg(c.p + 2 * c.pl), __ldg(c.p + 3 * c.pl)};
+  Cons r{load_coherent(c.p), load_coherent(c.p + c.pl), load_coherent(c.p + 2 * c.pl), load_coherent(c.p + 3 * c.pl)};
   if (c.flip) r.my = -r.my;
   return r;
 }
@@ -453,19 +467,19 @@ fv_step_kernel(const EcgFvParams P, const double* __restrict__ u, double* __rest
     {
       const double* F = s_fx;
       const double* G = s_fy;
-      const double o0 = __ldg(u + o);
+      const double o0 = load_coherent(u + o);
       n.rho = o0 - dt * ((F[xl + 1] - F[xl]) * inv_dx + (G[yb + TX] - G[yb]) * inv_dy);
       F += S::NFX;
       G += S::NFY;
-      const double o1 = __ldg(u + o + pl);
+      const double o1 = load_coherent(u + o + pl);
       n.mx = o1 - dt * ((F[xl + 1] - F[xl]) * inv_dx + (G[yb + TX] - G[yb]) * inv_dy);
       F += S::NFX;
       G += S::NFY;
-      const double o2 = __ldg(u + o + 2 * pl);
+      const double o2 = load_coherent(u + o + 2 * pl);
       n.my = o2 - dt * ((F[xl + 1] - F[xl]) * inv_dx + (G[yb + TX] - G[yb]) * inv_dy);
       F += S::NFX;
       G += S::NFY;
-      const double o3 = __ldg(u + o + 3 * pl);
+      const double o3 = load_coherent(u + o + 3 * pl);
       n.E = o3 - dt * ((F[xl + 1] - F[xl]) * inv_dx + (G[yb + TX] - G[yb]) * inv_dy);
     }
     out[o] = n.rho;
@@ -834,12 +848,12 @@ __global__ void init_state_kernel(const EcgFvParams P, const EcgProblem pr, doub
 // 400x4 walking the whole box and solving the Riemann problem for every ghost
 // cell took 13.5 us a step, the ring alone with the star state known 3 us.
 __global__ void ghost_box_kernel(const EcgFvParams P, const EcgProblem pr, const double* __restrict__ u, double time,
-                                 const EcgStepStats* __restrict__ stats, int k, double* __restrict__ out,
+                                 const EcgStepStats* stats, int k, double* __restrict__ out,
                                  long long opitch, long long oplane, int only_ring)
 {
-  loop_ready();
   loop_wait();
-  if (stats != nullptr) time = stats[k].t;
+  loop_ready();  // (before the wait it brings 0.5 % on 400x4, within the noise of the runs)
+  if (stats != nullptr) time = load_coherent(&stats[k].t);
   const int nx = P.g.nx, ny = P.g.ny, W = nx + 4, H = ny + 4;
   const int n = only_ring ? 4 * W + 4 * ny : W * H;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
