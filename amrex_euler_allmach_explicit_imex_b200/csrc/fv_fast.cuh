@@ -357,7 +357,7 @@ static __device__ __noinline__ Cons xie_f(const Prim l, const Prim r, int axis, 
 // xie_f without branches: the flux of a face whose states take none of
 // xie_f's exits (sound speeds on the rsqrt path, ordered wave speeds, and for
 // a subsonic face no degenerate denominator, densities and Roe sound speed on
-// the fast path and a finite result).  `fallback` marks the faces xie_f must
+// the fast path) and whose result is finite.  `fallback` marks the faces xie_f must
 // evaluate instead (the caller does so after one warp vote; the thresholds
 // here are a shade wider than xie_f's, which decides).  No face that stays is
 // degenerate for the HLLC test: its middle speed is this one.
@@ -416,9 +416,10 @@ __device__ __forceinline__ Cons xie_core(const Prim& l, const Prim& r, int axis,
   const double FE = ss * (rs * e + (ss - un) * fma(p, inv_sd, rss) + ps) + 0.5 * bp * v2h;
   const bool sub_exit = fabs(ad) <= kTiny || fabs(sl - ss0) <= kTiny || fabs(sr - ss0) <= kTiny ||
                         fabs(al) <= kTiny || fabs(ar) <= kTiny || !pos_normal_range(rr) || !(l.rho > 0.0) ||
-                        !(cl > kTiny) || !(cr > kTiny) || !(c2 > 1.01e-24) || !(c2 < 1.0e300) ||
-                        !isfinite(FE + mn + mt);
-  fallback = bl || br || !ordered || (!supersonic && sub_exit);
+                        !(cl > kTiny) || !(cr > kTiny) || !(c2 > 1.01e-24) || !(c2 < 1.0e300);
+  // (a supersonic face too: Roe averages off the number range, or a wave speed
+  // that rounds to the flow's, leave a NaN where xie_f returns the upwind flux)
+  fallback = bl || br || !ordered || (!supersonic && sub_exit) || !isfinite(FE + mn + mt);
   return Cons{rss + bp, axis == 0 ? mn : mt, axis == 0 ? mt : mn, FE};
 }
 
