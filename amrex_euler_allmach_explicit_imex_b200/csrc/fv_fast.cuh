@@ -197,9 +197,9 @@ __device__ __forceinline__ double mach_limit(double sp2l, double icl, double sp2
 // whose sound speeds the flux shares) without branches or votes: the flux of
 // faces whose sound speeds are on the rsqrt path and whose star state is not
 // degenerate.  `fallback` marks the faces that hllc_f must recompute
-// (degenerate star state, a sound speed off the rsqrt path or, for LM, below
-// the floor of the Mach numbers), so that a warp evaluates two faces back to
-// back and repairs them after one vote.
+// (degenerate star state, a wave speed equal to its side's velocity, a sound
+// speed off the rsqrt path or, for LM, below the floor of the Mach numbers), so
+// that a warp evaluates two faces back to back and repairs them after one vote.
 //
 // The star flux F_K + s_K (U*_K - U_K) is evaluated in its collapsed form: by
 // the jump conditions across s_K it equals
@@ -248,6 +248,10 @@ __device__ __forceinline__ Cons hllc_core(const Prim& ql, const Prim& qr, int ax
   const double ps = supersonic ? p : 0.5 * (fma(al, sm0 - unl, ql.p) + fma(ar, sm0 - unr, qr.p));
   const double inv_sd = frcp(s - sm);
   const double d = s - un;
+  // a supersonic side whose wave speed rounds to its own velocity (cold flow)
+  // has no quotient d / (s - sm): hllc_f returns its physical flux.  (On the
+  // bit pattern, beside the FP64 pipe.)
+  fallback = fallback || (__double2hiint(d) << 1) == 0;
   const double m = rho * d * inv_sd * sm;
   const double E = fma(p, inv_gm1, 0.5 * rho * fma(un, un, ut * ut));
   const double es = (d * E - p * un + ps * sm) * inv_sd;
