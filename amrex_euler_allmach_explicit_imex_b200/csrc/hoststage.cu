@@ -12,98 +12,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
-#include <condition_variable>
 #include <cstring>
 #include <functional>
-#include <mutex>
 #include <string>
 #include <thread>
-#include <vector>
 
+#include "copypool.h"
 #include "ctx.h"
-
-// A fixed set of host threads that run the n tasks of one job together with
-// the calling thread; run() returns when every task is done and no thread
-// holds the job any more (the job lives on run()'s stack).
-class CopyPool {
- public:
-  explicit CopyPool(int workers)
-  {
-    for (int w = 0; w < workers; ++w) threads_.emplace_back([this] { loop(); });
-  }
-  ~CopyPool()
-  {
-    {
-      std::lock_guard<std::mutex> lock(mu_);
-      stop_ = true;
-    }
-    cv_.notify_all();
-    for (auto& t : threads_) t.join();
-  }
-  void run(int n, const std::function<void(int)>& f)
-  {
-    Job job;
-    job.f = &f;
-    job.n = n;
-    {
-      std::lock_guard<std::mutex> lock(mu_);
-      job_ = &job;
-      ++gen_;
-    }
-    cv_.notify_all();
-    const int mine = drain(job);
-    std::unique_lock<std::mutex> lock(mu_);
-    job.done += mine;
-    job_ = nullptr;  // no thread takes it from here on
-    done_cv_.wait(lock, [&] { return job.done == job.n && job.users == 0; });
-  }
-
- private:
-  struct Job {
-    const std::function<void(int)>* f = nullptr;
-    int n = 0;
-    std::atomic<int> next{0};
-    int done = 0;   // tasks finished (under mu_)
-    int users = 0;  // worker threads holding the job (under mu_)
-  };
-  static int drain(Job& j)
-  {
-    int k, count = 0;
-    while ((k = j.next.fetch_add(1)) < j.n) {
-      (*j.f)(k);
-      ++count;
-    }
-    return count;
-  }
-  void loop()
-  {
-    unsigned long long seen = 0;
-    for (;;) {
-      Job* j = nullptr;
-      {
-        std::unique_lock<std::mutex> lock(mu_);
-        cv_.wait(lock, [&] { return stop_ || gen_ != seen; });
-        if (stop_) return;
-        seen = gen_;
-        j = job_;
-        if (!j) continue;
-        ++j->users;
-      }
-      const int count = drain(*j);
-      std::lock_guard<std::mutex> lock(mu_);
-      j->done += count;
-      --j->users;
-      if (j->done == j->n && j->users == 0) done_cv_.notify_all();
-    }
-  }
-  std::vector<std::thread> threads_;
-  std::mutex mu_;
-  std::condition_variable cv_, done_cv_;
-  Job* job_ = nullptr;
-  unsigned long long gen_ = 0;
-  bool stop_ = false;
-};
 
 struct HostStage {
   double* in = nullptr;   // pinned: what crosses to the device
