@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -51,8 +52,9 @@ struct ecg_batch {
   int ntiles = 0, grid = 0;
   long long launches = 0;              // launches so far (multiple of 3 between runs)
   cudaGraphExec_t graph = nullptr;
-  HostStage* stage = nullptr;          // pinned staging of large pageable boxes
-  cudaEvent_t band[4] = {};
+  size_t unstaged = 0;                 // bytes of large pageable boxes that crossed without the shared bands
+  std::shared_ptr<BandRing> ring;      // held from the first such box on
+  cudaEvent_t band[kBands] = {};
 
   bool ok(cudaError_t e, const char* what)
   {
@@ -63,7 +65,6 @@ struct ecg_batch {
   ~ecg_batch()
   {
     if (graph) cudaGraphExecDestroy(graph);
-    host_stage_destroy(stage);
     for (cudaEvent_t e : band)
       if (e) cudaEventDestroy(e);
     cudaFree(arena);
@@ -218,60 +219,32 @@ ecg_status uploaded(ecg_batch* b, int s)
   return ECG_OK;
 }
 
-constexpr long long kStagedCells = 32768;  // 1 MB: below it the stage's hand-overs cost what they save
+constexpr long long kStagedCells = 32768;  // 1 MB: below it the hand-overs cost what they save
+// The shared bands cost 3 to 6 ms to make and give back, about what they save on
+// this many bytes: a batch takes them up once it has moved as much without.  Build,
+// upload, one step, download of 3 solves of 1024x1024: 31 ms (40 to 50 without the
+// bands, 54 to 66 with a stage of the batch's own), of 8 of 512x512 27 (34, 32); the
+// transfers of 64 of 256x256 once more: 9.5 ms up, 8.8 down (14.8, 14 to 70; 10, 9.9).
+constexpr size_t kStagedBytes = 32u << 20;
 
-// The batch's stage for one direction, sized for its largest solve; null when
-// it cannot be had.
-double* batch_stage(ecg_batch* b, bool upload)
+// The shared bands and this batch's events, or null when they cannot be had.
+BandRing* batch_ring(ecg_batch* b)
 {
-  size_t most = 0;
-  for (const EcgBatchSolve& S : b->solves) most = std::max(most, 4 * static_cast<size_t>(S.p.g.nx) * S.p.g.ny);
-  b->stage = host_stage_sized(b->stage, most, upload);
-  return upload ? host_stage_in(b->stage) : host_stage_out(b->stage);
-}
-
-// One solve's state between its pageable host box (offset to cell (0, 0)) and
-// the device, in bands of rows: the host threads copy one band while another
-// crosses.
-bool transfer_staged(ecg_batch* b, const EcgBatchSolve& S, double* dev, double* stage, double* host, int64_t jstride,
-                     int64_t nstride, bool upload)
-{
-  constexpr int kBands = 4;
-  if (!b->ok(cudaSetDevice(b->device), "device")) return false;  // the events' device
-  const int nx = S.p.g.nx, ny = S.p.g.ny, nb = std::min(kBands, ny);
-  const size_t plane = static_cast<size_t>(nx) * ny;
-  auto row0 = [&](int k) { return static_cast<int>(static_cast<long long>(ny) * k / nb); };
-  auto cross = [&](int k) {
-    for (int n = 0; n < 4; ++n) {
-      double* st = stage + n * plane + static_cast<size_t>(row0(k)) * nx;
-      double* d = dev + n * S.p.g.plane + static_cast<long long>(row0(k)) * S.p.g.pitch;
-      const size_t w = sizeof(double) * nx, pitch = sizeof(double) * S.p.g.pitch;
-      const int rows = row0(k + 1) - row0(k);
-      const cudaError_t e = upload ? cudaMemcpy2DAsync(d, pitch, st, w, w, rows, cudaMemcpyHostToDevice, b->stream)
-                                   : cudaMemcpy2DAsync(st, w, d, pitch, w, rows, cudaMemcpyDeviceToHost, b->stream);
-      if (!b->ok(e, upload ? "upload" : "download")) return false;
+  if (!b->ring) b->ring = band_ring();
+  if (b->ring && !b->band[kBands - 1]) {
+    DeviceGuard guard;
+    bool good = guard.enter(b->device) == cudaSuccess;
+    for (cudaEvent_t& e : b->band)
+      if (good && !e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        e = nullptr;
+        good = false;
+      }
+    if (!good) {
+      cudaGetLastError();
+      return nullptr;
     }
-    return true;
-  };
-  auto copy = [&](int k) {
-    host_stage_copy(b->stage, stage, host, jstride, nstride, nx, ny, row0(k), row0(k + 1), upload);
-  };
-  if (upload) {
-    for (int k = 0; k < nb; ++k) {
-      copy(k);
-      if (!cross(k)) return false;
-    }
-    return b->ok(cudaStreamSynchronize(b->stream), "sync");
   }
-  for (int k = 0; k < kBands; ++k)
-    if (!b->band[k] && !b->ok(cudaEventCreateWithFlags(&b->band[k], cudaEventDisableTiming), "event")) return false;
-  for (int k = 0; k < nb; ++k)
-    if (!cross(k) || !b->ok(cudaEventRecord(b->band[k], b->stream), "event")) return false;
-  for (int k = 0; k < nb; ++k) {
-    if (!b->ok(cudaEventSynchronize(b->band[k]), "sync")) return false;
-    copy(k);
-  }
-  return true;
+  return b->ring.get();
 }
 
 ecg_status transfer(ecg_batch* b, int s, double* host, const double* hostc, int32_t lo_x, int32_t lo_y,
@@ -283,14 +256,22 @@ ecg_status transfer(ecg_batch* b, int s, double* host, const double* hostc, int3
   if (lo_x > 0 || lo_y > 0 || jstride < nx - lo_x || nstride < jstride * (ny - lo_y)) return ECG_ERR_BAD_ARG;
   const int64_t off = static_cast<int64_t>(-lo_x) + static_cast<int64_t>(-lo_y) * jstride;
   double* dev = upload ? S.u[0] : S.u[b->steps[s] & 1];
-  // Large solves cross pageable memory through the batch's pinned stage, as a
-  // context's state does: the driver's own staging brings 3 GB/s into fresh pages
-  // here (64 solves, 164 MB: 58 ms, 25 ms staged).
-  if (static_cast<long long>(nx) * ny >= kStagedCells && host_pageable(upload ? hostc : host))
-    if (double* stage = batch_stage(b, upload))
-      return transfer_staged(b, S, dev, stage, (upload ? const_cast<double*>(hostc) : host) + off, jstride, nstride, upload)
-                 ? (upload ? uploaded(b, s) : ECG_OK)
-                 : ECG_ERR_CUDA;
+  // Large solves cross pageable memory through the shared pinned bands, as a
+  // context's state does through its stage: the driver's own staging brings 3 GB/s
+  // into fresh pages here.
+  if (static_cast<long long>(nx) * ny >= kStagedCells && host_pageable(upload ? hostc : host)) {
+    BandRing* ring = b->unstaged >= kStagedBytes ? batch_ring(b) : nullptr;
+    if (!ring) b->unstaged += 4 * sizeof(double) * nx * ny;
+    cudaError_t e = cudaSuccess;
+    const BandResult r = ring ? band_transfer(*ring, (upload ? const_cast<double*>(hostc) : host) + off, jstride, nstride,
+                                              dev, S.p.g.pitch, S.p.g.plane, nx, ny, upload, b->stream, b->band, e)
+                              : BandResult::kNotTaken;
+    if (r == BandResult::kFailed) {
+      b->ok(e, upload ? "upload" : "download");
+      return ECG_ERR_CUDA;
+    }
+    if (r == BandResult::kDone) return upload ? uploaded(b, s) : ECG_OK;
+  }
   for (int n = 0; n < 4; ++n) {
     double* d = dev + n * S.p.g.plane;
     cudaError_t e;

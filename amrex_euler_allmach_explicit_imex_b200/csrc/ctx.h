@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -106,7 +107,6 @@ bool fetch_fused(ecg_ctx* c);
 // the context's pinned staging buffers
 bool host_pageable(const void* p);
 HostStage* host_stage(ecg_ctx* c);  // null when the pinned buffers cannot be allocated (c->err set)
-HostStage* host_stage_sized(HostStage* s, size_t doubles, bool to_device);  // s or a new one, its buffer for the direction made
 void host_stage_destroy(HostStage* s);
 double* host_stage_in(HostStage* s);
 double* host_stage_out(HostStage* s);
@@ -114,6 +114,38 @@ double* host_stage_out(HostStage* s);
 // and the compact stage, on the staging threads
 void host_stage_copy(HostStage* s, double* stage, double* host, int64_t jstride, int64_t nstride, int nx, int ny,
                      int r0, int r1, bool to_stage);
+// Large pageable boxes of a batch: a ring of pinned bands shared by the batches
+// of the process.
+struct BandRing;
+constexpr int kBands = 4;
+enum class BandResult { kDone, kFailed, kNotTaken };
+std::shared_ptr<BandRing> band_ring();  // null when it cannot be had
+// the 4 planes of nx x ny between the caller's box (offset to cell (0, 0)) and
+// the device, on `stream`, with kBands events of its device; returns when the
+// last byte has arrived, or at once with kNotTaken when the ring is in use or a
+// row does not fit a band
+BandResult band_transfer(BandRing& ring, double* host, int64_t jstride, int64_t nstride, double* dev, long long pitch,
+                         long long plane, int nx, int ny, bool upload, cudaStream_t stream, cudaEvent_t* event,
+                         cudaError_t& err);
+
+// Restores the caller's current device on every exit path.
+struct DeviceGuard {
+  int prev = -1;
+  bool switched = false;
+  cudaError_t enter(int dev)
+  {
+    cudaError_t e = cudaGetDevice(&prev);
+    if (e != cudaSuccess) return e;
+    if (prev == dev) return cudaSuccess;
+    e = cudaSetDevice(dev);
+    switched = e == cudaSuccess;
+    return e;
+  }
+  ~DeviceGuard()
+  {
+    if (switched) cudaSetDevice(prev);
+  }
+};
 
 // imex.cu
 void imex_free(ecg_ctx* c);

@@ -96,25 +96,6 @@ ecg_status scratch_on(int dev, unsigned char** out, int* sms, char* err, int32_t
   return ECG_OK;
 }
 
-// Restores the caller's current device on every exit path.
-struct DeviceGuard {
-  int prev = -1;
-  bool switched = false;
-  cudaError_t enter(int dev)
-  {
-    cudaError_t e = cudaGetDevice(&prev);
-    if (e != cudaSuccess) return e;
-    if (prev == dev) return cudaSuccess;
-    e = cudaSetDevice(dev);
-    switched = e == cudaSuccess;
-    return e;
-  }
-  ~DeviceGuard()
-  {
-    if (switched) cudaSetDevice(prev);
-  }
-};
-
 ecg_status fail(char* err, int32_t len, ecg_status st, const char* what, cudaError_t e)
 {
   char msg[256];
