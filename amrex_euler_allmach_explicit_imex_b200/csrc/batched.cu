@@ -124,7 +124,7 @@ bool seed_solve(ecg_batch* b, int s)
   return b->ok(ecg_fast_ops.init_stats(st, 3, 0.0, b->stream), "init stats") &&
          b->ok(ecg_fast_ops.init_state_stats(b->d_state_stats, b->stream), "init state stats") &&
          b->ok(ecg_fast_ops.state_reduce(S.p, S.u[0], 0, b->d_state_stats, b->stream), "reduce") &&
-         b->ok(ecg_fast_ops.seed_stats(st, b->d_state_stats, b->stream), "seed");
+         b->ok(ecg_fast_ops.seed_stats(st, b->d_state_stats, nullptr, EcgLoopLimits{}, b->stream), "seed");
 }
 
 // Times every tile shape for a few launches on a scratch copy of the batch

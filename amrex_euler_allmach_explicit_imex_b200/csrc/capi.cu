@@ -247,6 +247,7 @@ ecg_ctx::~ecg_ctx()
   cudaFree(d_stats);
   cudaFree(d_state_stats);
   cudaFree(d_star);
+  cudaFree(d_limits);
   cudaFree(adj_gq);
   cudaFree(adj_stats);
   cudaFreeHost(h_stats);
@@ -416,6 +417,7 @@ ecg_status ecg_create(ecg_ctx** out, const ecg_run_config* cfg, const ecg_gpu_op
   c->stats_cap = ecg_ctx::kChunk + 1;  // >= 3 host-mode slots
   ok = ok && cuda_ok(c, cudaMalloc(&c->d_stats, sizeof(EcgStepStats) * c->stats_cap), "alloc stats");
   ok = ok && cuda_ok(c, cudaMallocHost(&c->h_stats, sizeof(EcgStepStats) * c->stats_cap), "alloc host stats");
+  ok = ok && cuda_ok(c, cudaMalloc(&c->d_limits, sizeof(EcgLoopLimits)), "alloc limits");
   ok = ok && cuda_ok(c, cudaMalloc(&c->d_state_stats, sizeof(EcgStateStats)), "alloc state stats");
   ok = ok && cuda_ok(c, cudaMallocHost(&c->h_state_stats, sizeof(EcgStateStats)), "alloc host state stats");
   // the exact ghosts of a Toro problem sample one Riemann solution: its star
@@ -914,30 +916,28 @@ static ecg_status run_explicit(ecg_ctx* c, int32_t max_step, double stop_time, e
   const int eq79 = 0;
   if (!cuda_ok(c, c->ops->state_reduce(p, c->cur_state(), eq79, c->d_state_stats, c->stream), "reduce"))
     return ECG_ERR_CUDA;
-  if (!cuda_ok(c, c->ops->seed_stats(c->d_stats, c->d_state_stats, c->stream), "seed")) return ECG_ERR_CUDA;
+  if (!cuda_ok(c, c->ops->seed_stats(c->d_stats, c->d_state_stats, c->d_limits, EcgLoopLimits{stop_time, static_cast<double>(max_step)}, c->stream),
+               "seed"))
+    return ECG_ERR_CUDA;
   for (;;) {
     EcgDtCtl ctl;
     std::memset(&ctl, 0, sizeof(ctl));
     ctl.device_dt = 1;
-    ctl.max_step = max_step;
+    ctl.limits = c->d_limits;
     ctl.count_degenerate = c->cfg.riemann != ECG_RIEMANN_RUSANOV;
     ctl.reset_slot = -1;
     ctl.cfl = c->cfg.cfl;
-    ctl.stop_time = stop_time;
-    // capture (or reuse) the chunk graph for this buffer parity and step base;
-    // no launches past the step limit (a stopped step is a launch all the same)
+    // capture (or reuse) the chunk graph for this buffer parity; no launches past
+    // the step limit (a stopped step is a launch all the same)
     const int nodes = std::max(1, std::min(K, max_step - steps));
     ecg_ctx::Graph* gr = nullptr;
     for (auto& g : c->graphs) {
-      if (g.cur == c->cur && g.nodes == nodes && g.max_step == max_step && g.stop_time == stop_time) gr = &g;
+      if (g.cur == c->cur && g.nodes == nodes) gr = &g;
     }
     if (!gr) {
-      c->graphs.push_back(ecg_ctx::Graph());
-      gr = &c->graphs.back();
-      gr->cur = c->cur;
-      gr->nodes = nodes;
-      gr->max_step = max_step;
-      gr->stop_time = stop_time;
+      ecg_ctx::Graph g;
+      g.cur = c->cur;
+      g.nodes = nodes;
       cudaGraph_t graph;
       if (!cuda_ok(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "capture")) return ECG_ERR_CUDA;
       for (int k = 0; k < nodes; ++k) {
@@ -951,9 +951,11 @@ static ecg_status run_explicit(ecg_ctx* c, int32_t max_step, double stop_time, e
       }
       const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
       if (!cuda_ok(c, ce, "end capture")) return ECG_ERR_CUDA;
-      const cudaError_t ie = cudaGraphInstantiate(&gr->exec, graph, 0);
+      const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
       cudaGraphDestroy(graph);
       if (!cuda_ok(c, ie, "instantiate")) return ECG_ERR_CUDA;
+      c->graphs.push_back(g);
+      gr = &c->graphs.back();
     }
     if (!cuda_ok(c, cudaGraphLaunch(gr->exec, c->stream), "graph launch")) return ECG_ERR_CUDA;
     if (!cuda_ok(c, cudaMemcpyAsync(c->h_stats, c->d_stats, sizeof(EcgStepStats) * (nodes + 1), cudaMemcpyDeviceToHost,

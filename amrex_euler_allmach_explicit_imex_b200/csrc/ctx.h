@@ -60,11 +60,10 @@ struct ecg_ctx {
   struct Graph {
     int cur = 0;
     int nodes = 0;  // steps in the graph
-    int max_step = 0;
-    double stop_time = 0.0;
     cudaGraphExec_t exec = nullptr;
   };
-  std::vector<Graph> graphs;
+  std::vector<Graph> graphs;                // at most two (buffer parities) for each node count up to kChunk
+  EcgLoopLimits* d_limits = nullptr;        // of the run in progress
 
   // slab of a grid split along x (ecg_create_slab): x sides whose ghost
   // columns come from the neighbour slabs, and the caller's halo blocks

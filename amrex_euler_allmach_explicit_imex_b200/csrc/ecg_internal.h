@@ -101,16 +101,23 @@ struct EcgStepStats {
   int step;                          // steps taken before the step reading this record
 };
 
+// Limits of a device loop.  They stand in device memory, not in the launches, so
+// that a captured graph serves every run.
+struct alignas(16) EcgLoopLimits {
+  double stop_time;
+  double max_step;
+};
+
 // dt control of one explicit launch.
 struct EcgDtCtl {
   int device_dt;      // 0: use dt/time below; 1: compute dt from stats[read_slot] like compute_euler_dt
-  int max_step;       // device mode: loop step limit
   int count_degenerate;
   int read_slot;      // device mode: record of the state this launch advances
   int acc_slot;       // record receiving the reductions of the new state
   int reset_slot;     // record this launch re-initialises for the next one (-1: none)
   double dt, time;    // host mode
-  double cfl, stop_time;
+  double cfl;
+  const EcgLoopLimits* limits;  // device mode
 };
 
 // One solve of a batch (batched.cu).  u[k & 1] holds the state after k
@@ -157,7 +164,8 @@ struct EcgStencilOps {
                            int only_ring, cudaStream_t s);
   cudaError_t (*init_stats)(EcgStepStats* stats, int n, double t0, cudaStream_t s);
   cudaError_t (*init_state_stats)(EcgStateStats* st, cudaStream_t s);
-  cudaError_t (*seed_stats)(EcgStepStats* stats, const EcgStateStats* st, cudaStream_t s);
+  cudaError_t (*seed_stats)(EcgStepStats* stats, const EcgStateStats* st, EcgLoopLimits* to, EcgLoopLimits limits,
+                            cudaStream_t s);  // and the loop's limits to *to unless null
   cudaError_t (*init_state)(const EcgFvParams& p, const EcgProblem& pr, double* u, cudaStream_t s);
   cudaError_t (*riemann_star)(const EcgProblem& pr, double* out, cudaStream_t s);
 };
