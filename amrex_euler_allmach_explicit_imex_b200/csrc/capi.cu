@@ -395,7 +395,8 @@ ecg_status ecg_create(ecg_ctx** out, const ecg_run_config* cfg, const ecg_gpu_op
   c->grid.inv_dy = 1.0 / c->grid.dy;
   c->grid.plo_x = cfg->prob_lo[0];
   c->grid.plo_y = cfg->prob_lo[1];
-  // kernel choice: 0 default (column strips), 2 column strips with faces one at a time,
+  // kernel choice: 0 default (column strips; for the HLLC-P flux tiles where
+  // they are the faster), 2 column strips with faces one at a time,
   // 1 square 16x16 tile (fast build), 8 or 16: 32xTY tile
   c->tile_y = (o.tile_y == 1 || o.tile_y == 2 || o.tile_y == 3 || o.tile_y == 8 || o.tile_y == 16) ? o.tile_y : 0;
   const size_t sbytes = sizeof(double) * 4 * c->grid.plane;

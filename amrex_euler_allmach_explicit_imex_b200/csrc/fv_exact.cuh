@@ -1,7 +1,8 @@
 // The arithmetic of the column strips (fv_march.cuh) in the exact build: the
 // names the fast build defines in fv_fast.cuh, with the reference's IEEE
-// expressions (ecg_device.cuh).  Included inside the ecg_exact namespace of
-// stencil.cuh.  A face flux takes its branches as it goes; `fallback` then
+// expressions (ecg_device.cuh), for the fluxes the exact build's strips
+// evaluate (HLLC-P stays on the tiles).  Included inside the ecg_exact namespace
+// of stencil.cuh.  A face flux takes its branches as it goes; `fallback` then
 // only reports a degenerate star state, whose face the strip evaluates once
 // more for its count.
 namespace fast {
@@ -10,7 +11,6 @@ __device__ __forceinline__ double frcp(double b) { return 1.0 / b; }
 __device__ __forceinline__ Prim to_prim_f(const Cons& c, double g) { return to_prim(c, g); }
 __device__ __forceinline__ double slope_f(double bk, double fw, int lim) { return limited_slope(bk, fw, lim); }
 __device__ __forceinline__ double fsound_w(double rho, double p, double g) { return sqrt(g * p / rho); }
-__device__ __forceinline__ double pratio_f(double pl, double pr) { return pressure_ratio(pl, pr); }
 
 __device__ __forceinline__ Cons rusanov_f(const Prim& l, const Prim& r, int axis, double g, double)
 {
@@ -31,15 +31,6 @@ __device__ __forceinline__ Cons hllc_core(Prim l, Prim r, int axis, double g, do
 {
   if (LM) lowmach_correct(l, r, g);
   return hllc_flux(l, r, axis, g, fallback);
-}
-__device__ __forceinline__ Cons xie_f(const Prim& l, const Prim& r, int axis, double g, double, double sensor, bool& deg)
-{
-  return xie_flux(l, r, axis, g, sensor, deg);
-}
-__device__ __forceinline__ Cons xie_core(const Prim& l, const Prim& r, int axis, double g, double, double sensor,
-                                         bool& fallback)
-{
-  return xie_flux(l, r, axis, g, sensor, fallback);
 }
 
 }  // namespace fast

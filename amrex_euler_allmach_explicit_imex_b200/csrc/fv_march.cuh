@@ -15,7 +15,8 @@
 // committed once per block.
 // Two forms: rows through shared memory (march_strip_staged, the default), and
 // rows j-1 .. j+2 in registers with the x-neighbours by warp shuffles
-// (march_strip, the fast build's tile_y 2 and 3).
+// (march_strip, the fast build's tile_y 2 and 3).  The HLLC-P flux takes the
+// strips in the fast build only, too.
 namespace march {
 
 #ifdef ECG_FAST_KERNEL
@@ -25,10 +26,6 @@ constexpr bool kExact = true;
 #endif
 constexpr int kLanes = 32;
 constexpr int kCells = 28;  // interior cells per warp strip
-
-struct Lane {
-  Prim q[4];  // rows j-1, j, j+1, j+2 of this lane's column
-};
 
 __device__ __forceinline__ double shup(double v) { return __shfl_up_sync(0xffffffffu, v, 1); }
 __device__ __forceinline__ double shdn(double v) { return __shfl_down_sync(0xffffffffu, v, 1); }
@@ -52,55 +49,42 @@ __device__ __forceinline__ Prim minus_half(const Prim& q, const Prim& s)
 }
 
 // One face on its own, every branch taken (the y-face below the first row of a
-// strip, and the faces the branch-free cores send back).
+// strip, and the faces the branch-free cores send back).  deg: HLLC fell back to
+// Rusanov.  sensor: of the HLLC-P flux, h^3 of the five faces' ratios.
 template <int RK>
-__device__ __forceinline__ Cons face_one(Prim l, Prim r, int axis, double g, double inv_gm1, bool& deg)
+__device__ __forceinline__ Cons face_one(Prim l, Prim r, int axis, double g, double inv_gm1, double sensor, bool& deg)
 {
   deg = false;
+#ifdef ECG_FAST_KERNEL
+  if (RK == ECG_RIEMANN_XIE_AM_HLLC_P) return fast::xie_f(l, r, axis, g, inv_gm1, sensor, deg);
+#endif
   if (RK == ECG_RIEMANN_RUSANOV) return fast::rusanov_f(l, r, axis, g, inv_gm1);
   if (RK == ECG_RIEMANN_LOWMACH_HLLC) fast::lowmach_f(l, r, g);
   return fast::hllc_f(l, r, axis, g, inv_gm1, deg);
 }
 
-// The x-face and the y-face of a row, evaluated back to back on the fast
-// path (independent instruction streams the scheduler can interleave); faces
-// that need the reference path (degenerate HLLC star state, sound speed off
-// the rsqrt path) are recomputed after one warp vote.  deg_*: HLLC fell back
-// to Rusanov on that face.  Returns whether the vote fired (the same on every
-// lane): deg_* can only be set then.
+// The face without branches; `b` marks one that face_one must evaluate instead.
 template <int RK>
-__device__ __forceinline__ bool face_pair(Prim xl, Prim xr, Prim yl, Prim yr, double g, double inv_gm1, Cons& fx,
-                                          Cons& fy, bool& deg_x, bool& deg_y)
+__device__ __forceinline__ Cons face_core(const Prim& l, const Prim& r, int axis, double g, double inv_gm1,
+                                          double sensor, bool& b)
 {
-  bool bx, by;
-  constexpr bool LM = RK == ECG_RIEMANN_LOWMACH_HLLC;
-  if (RK == ECG_RIEMANN_RUSANOV) {
-    fx = fast::rusanov_core(xl, xr, 0, g, inv_gm1, bx);
-    fy = fast::rusanov_core(yl, yr, 1, g, inv_gm1, by);
-  } else {
-    fx = fast::hllc_core<LM>(xl, xr, 0, g, inv_gm1, bx);
-    fy = fast::hllc_core<LM>(yl, yr, 1, g, inv_gm1, by);
-  }
-  deg_x = deg_y = false;
-  if (__any_sync(0xffffffffu, bx || by)) {
-    if (bx) fx = face_one<RK>(xl, xr, 0, g, inv_gm1, deg_x);
-    if (by) fy = face_one<RK>(yl, yr, 1, g, inv_gm1, deg_y);
-    return true;
-  }
-  return false;
+#ifdef ECG_FAST_KERNEL
+  if (RK == ECG_RIEMANN_XIE_AM_HLLC_P) return fast::xie_core(l, r, axis, g, inv_gm1, sensor, b);
+#endif
+  if (RK == ECG_RIEMANN_RUSANOV) return fast::rusanov_core(l, r, axis, g, inv_gm1, b);
+  return fast::hllc_core<RK == ECG_RIEMANN_LOWMACH_HLLC>(l, r, axis, g, inv_gm1, b);
 }
 
-// One face, repaired after a vote of its own (faces evaluated one after the other).
+// One face, repaired after a vote of its own.
 template <int RK>
-__device__ __forceinline__ Cons face_w(Prim l, Prim r, int axis, double g, double inv_gm1, bool& deg)
+__device__ __forceinline__ Cons face_voted(const Prim& l, const Prim& r, int axis, double g, double inv_gm1,
+                                           double sensor, bool& deg)
 {
   bool b;
-  constexpr bool LM = RK == ECG_RIEMANN_LOWMACH_HLLC;
-  Cons f = RK == ECG_RIEMANN_RUSANOV ? fast::rusanov_core(l, r, axis, g, inv_gm1, b)
-                                     : fast::hllc_core<LM>(l, r, axis, g, inv_gm1, b);
+  Cons f = face_core<RK>(l, r, axis, g, inv_gm1, sensor, b);
   deg = false;
   if (__any_sync(0xffffffffu, b)) {
-    if (b) f = face_one<RK>(l, r, axis, g, inv_gm1, deg);
+    if (b) f = face_one<RK>(l, r, axis, g, inv_gm1, sensor, deg);
   }
   return f;
 }
@@ -117,6 +101,33 @@ struct MarchAcc {
     nonfinite = degenerate = 0;
   }
 };
+
+#ifdef ECG_FAST_KERNEL
+struct Lane {
+  Prim q[4];  // rows j-1, j, j+1, j+2 of this lane's column
+};
+
+// The x-face and the y-face of a row, evaluated back to back on the fast
+// path (independent instruction streams the scheduler can interleave); faces
+// that need the reference path (degenerate HLLC star state, sound speed off
+// the rsqrt path) are recomputed after one warp vote.  deg_*: HLLC fell back
+// to Rusanov on that face.  Returns whether the vote fired (the same on every
+// lane): deg_* can only be set then.
+template <int RK>
+__device__ __forceinline__ bool face_pair(const Prim& xl, const Prim& xr, const Prim& yl, const Prim& yr, double g,
+                                          double inv_gm1, Cons& fx, Cons& fy, bool& deg_x, bool& deg_y)
+{
+  bool bx, by;
+  fx = face_core<RK>(xl, xr, 0, g, inv_gm1, 0.0, bx);
+  fy = face_core<RK>(yl, yr, 1, g, inv_gm1, 0.0, by);
+  deg_x = deg_y = false;
+  if (__any_sync(0xffffffffu, bx || by)) {
+    if (bx) fx = face_one<RK>(xl, xr, 0, g, inv_gm1, 0.0, deg_x);
+    if (by) fy = face_one<RK>(yl, yr, 1, g, inv_gm1, 0.0, deg_y);
+    return true;
+  }
+  return false;
+}
 
 // Advances the strip of 28 cells starting at column c0 over rows
 // [j0, min(j0 + H, ny)) from u into out.  Called by all 32 lanes of a warp
@@ -150,7 +161,7 @@ __device__ __forceinline__ void march_strip(const EcgFvParams& P, const double* 
   Cons gb;
   {
     bool deg;
-    gb = face_one<RK>(plus_half(L.q[1], sy_m1), minus_half(L.q[2], sy_cur), 1, g, inv_gm1, deg);
+    gb = face_one<RK>(plus_half(L.q[1], sy_m1), minus_half(L.q[2], sy_cur), 1, g, inv_gm1, 0.0, deg);
     if (count_deg && deg && cell_ok && j0 < ny) acc.degenerate += 1;
   }
   for (int j = j0; j < jend; ++j) {
@@ -175,8 +186,8 @@ __device__ __forceinline__ void march_strip(const EcgFvParams& P, const double* 
       voted = face_pair<RK>(plus_half(ql, sxl), minus_half(qc, sx), plus_half(qc, sy_cur), minus_half(L.q[2], sy_next),
                             g, inv_gm1, fl, gt, deg_x, deg_y);
     } else {
-      gt = face_w<RK>(plus_half(qc, sy_cur), minus_half(L.q[2], sy_next), 1, g, inv_gm1, deg_y);
-      fl = face_w<RK>(plus_half(ql, sxl), minus_half(qc, sx), 0, g, inv_gm1, deg_x);
+      gt = face_voted<RK>(plus_half(qc, sy_cur), minus_half(L.q[2], sy_next), 1, g, inv_gm1, 0.0, deg_y);
+      fl = face_voted<RK>(plus_half(ql, sxl), minus_half(qc, sx), 0, g, inv_gm1, 0.0, deg_x);
     }
     const Cons fr{shdn(fl.rho), shdn(fl.mx), shdn(fl.my), shdn(fl.E)};
     if (count_deg && voted) {
@@ -214,6 +225,7 @@ __device__ __forceinline__ void march_strip(const EcgFvParams& P, const double* 
     sy_cur = sy_next;
   }
 }
+#endif  // ECG_FAST_KERNEL
 
 // ---- the staged march: rows live in shared memory --------------------------
 //
@@ -251,6 +263,7 @@ __device__ __forceinline__ void cp_async_wait()
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+#ifdef ECG_FAST_KERNEL
 // The multiface sensor's pressure ratio (xie_pressure_ratio_from_states,
 // reconstruction_fluxes.hpp:390-397) of the x-face on this lane's left in a
 // row of which this lane holds the pressure pc: the face pressures of the
@@ -263,21 +276,12 @@ __device__ __forceinline__ double xface_ratio(double pc, bool second)
   return fast::pratio_f(fma(0.5, shup(s), pl), fma(-0.5, s, pc));
 }
 
-// xie_am_hllc_p flux of one face with sensor h^3 (reconstruction_fluxes.hpp:
-// 254-371, 390-440): the branch-free core, repaired by xie_f on the faces a
-// warp vote sends back.  deg: the HLLC degeneracy test of the face.
-__device__ __forceinline__ Cons face_xie(const Prim& l, const Prim& r, int axis, double g, double inv_gm1, double h,
-                                         bool& deg)
+__device__ __forceinline__ double sensor_of(double ratio)
 {
-  const double sensor = h * h * h;
-  bool fb;
-  Cons f = fast::xie_core(l, r, axis, g, inv_gm1, sensor, fb);
-  deg = false;
-  if (__any_sync(0xffffffffu, fb)) {
-    if (fb) f = fast::xie_f(l, r, axis, g, inv_gm1, sensor, deg);
-  }
-  return f;
+  const double h = clamp01(ratio);
+  return h * h * h;
 }
+#endif
 
 // Advances the strip as march_strip does.  The x- and the y-face of a row are
 // evaluated back to back on the branch-free cores; faces those send back are
@@ -295,8 +299,6 @@ __device__ __forceinline__ bool march_strip_staged(const EcgFvParams& P, const d
                                                    double* __restrict__ out, int c0, int j0, int H, Control control,
                                                    bool count_deg, MarchAcc& acc, StageRing& ring)
 {
-  constexpr bool XIE = RK == ECG_RIEMANN_XIE_AM_HLLC_P;
-  constexpr bool LM = RK == ECG_RIEMANN_LOWMACH_HLLC;
   const int lane = threadIdx.x & 31;
   const int x = c0 - 2 + lane;
   const int nx = P.g.nx, ny = P.g.ny;
@@ -402,7 +404,7 @@ __device__ __forceinline__ bool march_strip_staged(const EcgFvParams& P, const d
   cp_async_wait<kAhead>();
   Prim yp;  // row j's state at its upper y-face
   Cons gb;  // the y-face below row j
-  double yr_prev = 0.0, xr_cur = 0.0;  // XIE: pressure ratios of the y-face below row j, the x-face left of row j
+  double yr_prev = 0.0, xr_cur = 0.0;  // HLLC-P: pressure ratios of the y-face below row j, the x-face left of row j
   {
     const Prim q_m2 = convert(j0 - 2), q_m1 = convert(j0 - 1), qa = convert(j0), qb = convert(j0 + 1);
     const Prim sy_m1 = slope3<LIM>(q_m2, q_m1, qa, second);
@@ -410,19 +412,16 @@ __device__ __forceinline__ bool march_strip_staged(const EcgFvParams& P, const d
     const Prim yl = plus_half(q_m1, sy_m1), yr = minus_half(qa, s0);
     yp = plus_half(qa, s0);
     bool deg;
-    if constexpr (XIE) {
+#ifdef ECG_FAST_KERNEL
+    if constexpr (RK == ECG_RIEMANN_XIE_AM_HLLC_P) {
       yr_prev = fast::pratio_f(yl.p, yr.p);
       const double xm1 = xface_ratio<LIM>(q_m1.p, second);
       xr_cur = xface_ratio<LIM>(qa.p, second);
-      double m = yr_prev;
-      m = smin(m, xm1);
-      m = smin(m, shdn(xm1));
-      m = smin(m, xr_cur);
-      m = smin(m, shdn(xr_cur));
-      gb = face_xie(yl, yr, 1, g, inv_gm1, clamp01(m), deg);
-    } else {
-      gb = face_one<RK>(yl, yr, 1, g, inv_gm1, deg);
-    }
+      const double m = smin(smin(smin(smin(yr_prev, xm1), shdn(xm1)), xr_cur), shdn(xr_cur));
+      gb = face_voted<RK>(yl, yr, 1, g, inv_gm1, sensor_of(m), deg);
+    } else
+#endif
+      gb = face_one<RK>(yl, yr, 1, g, inv_gm1, 0.0, deg);
     if (count_deg && deg && cell_ok && j0 < ny) acc.degenerate += 1;
   }
   double* o = out + static_cast<long long>(j0) * P.g.pitch + (x < 0 ? 0 : (x < nx ? x : nx - 1));
@@ -435,12 +434,13 @@ __device__ __forceinline__ bool march_strip_staged(const EcgFvParams& P, const d
     __syncwarp();  // every lane's row j + 2 is in the rings
     bool bx, by;
     Cons gt, fl;
-    double mx = 0.0, my = 0.0;  // XIE: the sensors of the two faces
+    double mx = 0.0, my = 0.0;  // HLLC-P: the sensors of the two faces
     {
       const Prim q1 = prim(j + 1, 0);
       const Prim sn = slope3<LIM>(prim(j, 0), q1, q2, second);
       const Prim yr = minus_half(q1, sn);
-      if constexpr (XIE) {
+#ifdef ECG_FAST_KERNEL
+      if constexpr (RK == ECG_RIEMANN_XIE_AM_HLLC_P) {
         // sensors: the y-face above, from its own ratio and the x-faces' left
         // and right of cell i in rows j and j+1; the x-face on the left, from
         // its own ratio and the y-faces' below and above cells i-1 and i
@@ -454,12 +454,9 @@ __device__ __forceinline__ bool march_strip_staged(const EcgFvParams& P, const d
         mx = clamp01(mx);
         yr_prev = yr_cur;
         xr_cur = xr_next;
-        gt = fast::xie_core(yp, yr, 1, g, inv_gm1, my * my * my, by);
-      } else if (RK == ECG_RIEMANN_RUSANOV) {
-        gt = fast::rusanov_core(yp, yr, 1, g, inv_gm1, by);
-      } else {
-        gt = fast::hllc_core<LM>(yp, yr, 1, g, inv_gm1, by);
       }
+#endif
+      gt = face_core<RK>(yp, yr, 1, g, inv_gm1, my * my * my, by);
       yp = plus_half(q1, sn);
     }
     {
@@ -467,22 +464,18 @@ __device__ __forceinline__ bool march_strip_staged(const EcgFvParams& P, const d
       const Prim sx = slope3<LIM>(prim(j, left), q0, prim(j, right), second);
       const Prim xp = plus_half(q0, sx), xr = minus_half(q0, sx);
       const Prim xl{shup(xp.rho), shup(xp.u), shup(xp.v), shup(xp.p)};
-      if constexpr (XIE) fl = fast::xie_core(xl, xr, 0, g, inv_gm1, mx * mx * mx, bx);
-      else if (RK == ECG_RIEMANN_RUSANOV) fl = fast::rusanov_core(xl, xr, 0, g, inv_gm1, bx);
-      else fl = fast::hllc_core<LM>(xl, xr, 0, g, inv_gm1, bx);
+      fl = face_core<RK>(xl, xr, 0, g, inv_gm1, mx * mx * mx, bx);
     }
     if (__any_sync(0xffffffffu, bx || by)) {
       Prim l, r;
       bool deg_x = false, deg_y = false;
       if (bx) {
         xstates(j, l, r);
-        if constexpr (XIE) fl = fast::xie_f(l, r, 0, g, inv_gm1, mx * mx * mx, deg_x);
-        else fl = face_one<RK>(l, r, 0, g, inv_gm1, deg_x);
+        fl = face_one<RK>(l, r, 0, g, inv_gm1, mx * mx * mx, deg_x);
       }
       if (by) {
         ystates(j, l, r);
-        if constexpr (XIE) gt = fast::xie_f(l, r, 1, g, inv_gm1, my * my * my, deg_y);
-        else gt = face_one<RK>(l, r, 1, g, inv_gm1, deg_y);
+        gt = face_one<RK>(l, r, 1, g, inv_gm1, my * my * my, deg_y);
       }
       if (count_deg) {
         // each face counts once per adjacent cell of this strip in the domain
@@ -553,15 +546,18 @@ constexpr int kStagedWarps = !kExact && (RK == ECG_RIEMANN_HLLC || RK == ECG_RIE
 // The register-loaded strips take at most 128 registers a thread (16 warps
 // per SM), measured faster than the 166-register schedule the paired faces get
 // unbounded.
-// STAGE: rows through the shared-memory ring (march_strip_staged), else
-// straight from global memory into registers (march_strip).
-template <int RK, int LIM, int WPB, bool PAIR, bool STAGE>
-__global__ void __launch_bounds__(WPB * 32, (STAGE ? kStagedWarps<RK> : 16) / WPB)
+// How the rows come and the faces are evaluated: through the shared-memory rings,
+// the two faces of a row together (march_strip_staged); straight from global
+// memory into registers (march_strip), the faces together or one after the other.
+enum class Form { kStaged, kPaired, kSingle };
+
+template <int RK, int LIM, int WPB, Form FORM>
+__global__ void __launch_bounds__(WPB * 32, (FORM == Form::kStaged ? kStagedWarps<RK> : 16) / WPB)
 fv_march_kernel(const EcgFvParams P, const double* __restrict__ u, double* __restrict__ out,
                 EcgStepStats* __restrict__ stats, const EcgDtCtl ctl, const int H)
 {
   __shared__ BlockRed<WPB * 32> red;
-  __shared__ StageRing ring[STAGE ? WPB : 1];
+  __shared__ StageRing ring[FORM == Form::kStaged ? WPB : 1];
   const int strip = blockIdx.x * WPB + (threadIdx.x >> 5);
   const int c0 = strip * kCells;
   const int j0 = (P.row_hi > 0 ? P.row_lo : 0) + blockIdx.y * H;
@@ -572,16 +568,20 @@ fv_march_kernel(const EcgFvParams P, const double* __restrict__ u, double* __res
   MarchAcc acc;
   acc.init();
   double dt;
-  if constexpr (STAGE) {
+  if constexpr (FORM == Form::kStaged) {
     // (a stop is the same for every warp of the launch)
     const bool go = c0 < P.g.nx ? march_strip_staged<RK, LIM>(P, u, out, c0, j0, H, control, ctl.count_degenerate != 0,
                                                               acc, ring[threadIdx.x >> 5])
                                 : control(dt);
     if (!go) return;
-  } else {
-    if (!control(dt)) return;
-    if (c0 < P.g.nx) march_strip<RK, LIM, PAIR>(P, u, out, c0, j0, H, dt, ctl.count_degenerate != 0, acc);
   }
+#ifdef ECG_FAST_KERNEL
+  if constexpr (FORM != Form::kStaged) {
+    if (!control(dt)) return;
+    if (c0 < P.g.nx)
+      march_strip<RK, LIM, FORM == Form::kPaired>(P, u, out, c0, j0, H, dt, ctl.count_degenerate != 0, acc);
+  }
+#endif
   loop_ready();
   block_commit<WPB * 32>(red, acc.kmax, acc.krho, acc.kp, acc.nonfinite, acc.degenerate, &stats[ctl.acc_slot]);
 }
@@ -613,7 +613,7 @@ inline int rows_per_warp(int rows, int blocks_x, long long slots)
 
 // Two warps a block: the strips of a row of blocks overhang the grid by at
 // most one (four a block: 2 % to 8 % of the warps idle on odd widths).
-template <int RK, int LIM, bool PAIR, bool STAGE>
+template <int RK, int LIM, Form FORM>
 cudaError_t launch_lim(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats, const EcgDtCtl& ctl,
                        cudaStream_t s)
 {
@@ -630,7 +630,7 @@ cudaError_t launch_lim(const EcgFvParams& p, const double* in, double* out, EcgS
     static int blocks_per_sm = 0;
     if (blocks_per_sm == 0) {
       int b = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fv_march_kernel<RK, LIM, WPB, PAIR, STAGE>, WPB * 32, 0) !=
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fv_march_kernel<RK, LIM, WPB, FORM>, WPB * 32, 0) !=
               cudaSuccess ||
           b < 1)
         b = 1;
@@ -639,18 +639,18 @@ cudaError_t launch_lim(const EcgFvParams& p, const double* in, double* out, EcgS
     H = rows_per_warp(rows, bx, static_cast<long long>(p.sm_count > 0 ? p.sm_count : 148) * blocks_per_sm);
   }
   const dim3 grid(bx, (rows + H - 1) / H);
-  return launch_loop(ctl.device_dt != 0, fv_march_kernel<RK, LIM, WPB, PAIR, STAGE>, grid, WPB * 32, 0, s, p, in, out,
+  return launch_loop(ctl.device_dt != 0, fv_march_kernel<RK, LIM, WPB, FORM>, grid, WPB * 32, 0, s, p, in, out,
                      stats, ctl, H);
 }
 
-template <int RK, bool PAIR, bool STAGE>
+template <int RK, Form FORM>
 cudaError_t launch_rk(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats, const EcgDtCtl& ctl,
                       cudaStream_t s)
 {
   switch (p.limiter) {
-    case ECG_LIMITER_MC: return launch_lim<RK, ECG_LIMITER_MC, PAIR, STAGE>(p, in, out, stats, ctl, s);
-    case ECG_LIMITER_VANLEER: return launch_lim<RK, ECG_LIMITER_VANLEER, PAIR, STAGE>(p, in, out, stats, ctl, s);
-    default: return launch_lim<RK, ECG_LIMITER_MINMOD, PAIR, STAGE>(p, in, out, stats, ctl, s);
+    case ECG_LIMITER_MC: return launch_lim<RK, ECG_LIMITER_MC, FORM>(p, in, out, stats, ctl, s);
+    case ECG_LIMITER_VANLEER: return launch_lim<RK, ECG_LIMITER_VANLEER, FORM>(p, in, out, stats, ctl, s);
+    default: return launch_lim<RK, ECG_LIMITER_MINMOD, FORM>(p, in, out, stats, ctl, s);
   }
 }
 
@@ -662,29 +662,29 @@ inline cudaError_t launch(const EcgFvParams& p, const double* in, double* out, E
                           const EcgDtCtl& ctl, cudaStream_t s)
 {
   switch (p.riemann) {
-    case ECG_RIEMANN_RUSANOV: return launch_rk<ECG_RIEMANN_RUSANOV, true, true>(p, in, out, stats, ctl, s);
-    case ECG_RIEMANN_LOWMACH_HLLC: return launch_rk<ECG_RIEMANN_LOWMACH_HLLC, true, true>(p, in, out, stats, ctl, s);
-    default: return launch_rk<ECG_RIEMANN_HLLC, true, true>(p, in, out, stats, ctl, s);
+    case ECG_RIEMANN_RUSANOV: return launch_rk<ECG_RIEMANN_RUSANOV, Form::kStaged>(p, in, out, stats, ctl, s);
+    case ECG_RIEMANN_LOWMACH_HLLC: return launch_rk<ECG_RIEMANN_LOWMACH_HLLC, Form::kStaged>(p, in, out, stats, ctl, s);
+    default: return launch_rk<ECG_RIEMANN_HLLC, Form::kStaged>(p, in, out, stats, ctl, s);
   }
 }
 #else
 template <int RK>
-cudaError_t launch_mode(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats, const EcgDtCtl& ctl,
-                        cudaStream_t s, bool pair, bool stage)
+cudaError_t launch_form(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats, const EcgDtCtl& ctl,
+                        cudaStream_t s, Form form)
 {
-  if (stage) return launch_rk<RK, true, true>(p, in, out, stats, ctl, s);
-  return pair ? launch_rk<RK, true, false>(p, in, out, stats, ctl, s) : launch_rk<RK, false, false>(p, in, out, stats, ctl, s);
+  switch (form) {
+    case Form::kStaged: return launch_rk<RK, Form::kStaged>(p, in, out, stats, ctl, s);
+    case Form::kPaired: return launch_rk<RK, Form::kPaired>(p, in, out, stats, ctl, s);
+    default: return launch_rk<RK, Form::kSingle>(p, in, out, stats, ctl, s);
+  }
 }
 
-// pair: evaluate the x- and y-face of a row together (one vote for both);
-// otherwise one after the other.  stage: paired faces, rows staged through
-// shared memory (march_strip_staged).
 inline cudaError_t launch(const EcgFvParams& p, const double* in, double* out, EcgStepStats* stats,
-                          const EcgDtCtl& ctl, cudaStream_t s, bool pair, bool stage)
+                          const EcgDtCtl& ctl, cudaStream_t s, Form form)
 {
   switch (p.riemann) {
-    case ECG_RIEMANN_RUSANOV: return launch_mode<ECG_RIEMANN_RUSANOV>(p, in, out, stats, ctl, s, pair, stage);
-    case ECG_RIEMANN_LOWMACH_HLLC: return launch_mode<ECG_RIEMANN_LOWMACH_HLLC>(p, in, out, stats, ctl, s, pair, stage);
+    case ECG_RIEMANN_RUSANOV: return launch_form<ECG_RIEMANN_RUSANOV>(p, in, out, stats, ctl, s, form);
+    case ECG_RIEMANN_LOWMACH_HLLC: return launch_form<ECG_RIEMANN_LOWMACH_HLLC>(p, in, out, stats, ctl, s, form);
     case ECG_RIEMANN_XIE_AM_HLLC_P: {
       // Staged strips carry the 5-face sensor along (2560x640 104 us against
       // the tile kernel's 150, 512x512 22.5 against 28.0, 128x128 7.2 against
@@ -695,11 +695,11 @@ inline cudaError_t launch(const EcgFvParams& p, const double* in, double* out, E
       // host step) takes the strips: the tile kernel steps whole grids only.
       const long long tiles = static_cast<long long>((p.g.nx + 15) / 16) * ((p.g.ny + 15) / 16);
       const long long sms = p.sm_count > 0 ? p.sm_count : 148;
-      if (stage && (p.row_hi > 0 || tiles <= sms || tiles > 3 * sms))
-        return launch_rk<ECG_RIEMANN_XIE_AM_HLLC_P, false, true>(p, in, out, stats, ctl, s);
+      if (form == Form::kStaged && (p.row_hi > 0 || tiles <= sms || tiles > 3 * sms))
+        return launch_rk<ECG_RIEMANN_XIE_AM_HLLC_P, Form::kStaged>(p, in, out, stats, ctl, s);
       return fast::launch(p, in, out, stats, ctl, s);
     }
-    default: return launch_mode<ECG_RIEMANN_HLLC>(p, in, out, stats, ctl, s, pair, stage);
+    default: return launch_form<ECG_RIEMANN_HLLC>(p, in, out, stats, ctl, s, form);
   }
 }
 

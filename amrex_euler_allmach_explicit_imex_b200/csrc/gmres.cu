@@ -419,7 +419,6 @@ __device__ __forceinline__ void warp_partial(double v, double* wpart)
 // the grid barrier (acc_settle), so every launch on the same inputs gives the
 // same bits.  Maxima are exact in any order and stay atomic.
 //
-//
 // Where every warp adds the sums it has (the small-block dot products), an
 // entry sits in a 128-byte line of its own (stride kAccLine): packed together,
 // some 60 entries from 148 blocks queue on four L2 lines (256x256 FP64: 22.5 us

@@ -543,9 +543,9 @@ cudaError_t launch_fv_step(const EcgFvParams& p, const double* in, double* out, 
   // through shared memory by cp.async (default: 57 us at 2560x640); 3: the
   // same with rows loaded into registers (70 us); 2: column-strip kernel,
   // faces one after the other; 1: square-tile kernel
-  if (tile_y == 0) return march::launch(p, in, out, stats, ctl, s, true, true);
-  if (tile_y == 3) return march::launch(p, in, out, stats, ctl, s, true, false);
-  if (tile_y == 2) return march::launch(p, in, out, stats, ctl, s, false, false);
+  if (tile_y == 0) return march::launch(p, in, out, stats, ctl, s, march::Form::kStaged);
+  if (tile_y == 3) return march::launch(p, in, out, stats, ctl, s, march::Form::kPaired);
+  if (tile_y == 2) return march::launch(p, in, out, stats, ctl, s, march::Form::kSingle);
   if (tile_y == 1) return fast::launch(p, in, out, stats, ctl, s);
 #else
   // 8 or 16: a 32xTY tile; else column strips, but for the XIE flux, whose

@@ -154,7 +154,9 @@ typedef struct ecg_gpu_options {
   int32_t tile_x;           /* column-strip kernel: rows each warp marches (0: sized to the waves of resident blocks) */
   int32_t tile_y;           /* explicit kernel: 0 default (column strips, x- and y-faces
                                evaluated together, rows staged through shared memory by
-                               cp.async), 3 the same with rows loaded into registers, 2
+                               cp.async; the HLLC-P flux on tiles in exact arithmetic, and
+                               in fast arithmetic on grids of one to three 16x16 tiles a
+                               multiprocessor), 3 the same with rows loaded into registers, 2
                                column strips with faces one at a time, 1 square 16x16
                                tiles (1 to 3: fast arithmetic), 8 or 16 the 32 x tile_y
                                tiles */
