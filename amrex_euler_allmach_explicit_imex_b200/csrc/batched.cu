@@ -220,12 +220,10 @@ ecg_status uploaded(ecg_batch* b, int s)
 }
 
 constexpr long long kStagedCells = 32768;  // 1 MB: below it the hand-overs cost what they save
-// The shared bands cost 3 to 6 ms to make and give back, about what they save on
-// this many bytes: a batch takes them up once it has moved as much without.  Build,
-// upload, one step, download of 3 solves of 1024x1024: 31 ms (40 to 50 without the
-// bands, 54 to 66 with a stage of the batch's own), of 8 of 512x512 27 (34, 32); the
-// transfers of 64 of 256x256 once more: 9.5 ms up, 8.8 down (14.8, 14 to 70; 10, 9.9).
-constexpr size_t kStagedBytes = 32u << 20;
+// The shared bands cost 3 to 6 ms to make and 2 to give back; they save 0.13 ms a
+// MB into fresh pages and 0.035 a MB up.  A batch takes them up once it has moved
+// the 64 MB that repay them without.
+constexpr size_t kStagedBytes = 64u << 20;
 
 // The shared bands and this batch's events, or null when they cannot be had.
 BandRing* batch_ring(ecg_batch* b)

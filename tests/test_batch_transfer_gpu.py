@@ -39,7 +39,7 @@ def _threads():
 def test_boxes_cross_unchanged(gpu, grid):
     cfgs, states = _states([grid, (256, 256)], 3)
     with api.Batch(cfgs) as b:
-        _round_trips(b, states, 1 + (40 << 20) // sum(2 * u.nbytes for u in states))
+        _round_trips(b, states, 1 + (72 << 20) // sum(2 * u.nbytes for u in states))
         _round_trips(b, states, 2)
 
 
